@@ -1,0 +1,666 @@
+// tdse_cluster.cu -- the TDSE propagation with one instance spread over a thread-block cluster.
+//
+// propagate_fp64_kernel and propagate_df64_kernel give an instance one CTA, so a batch smaller than
+// the GPU leaves SMs idle and a single call runs on one of 152.  Here a cluster of NC CTAs (1 to 16,
+// chosen by the host below) shares one instance: NC x 128 threads each own m contiguous sites, and
+// every table, psi and the sweep live in the cluster's shared memory for the whole pulse.
+//
+// A step is the partitioned solve of tdse_solver.cuh with three differences that keep the work per
+// thread small, because at few sites per thread the scans and reductions cost as much as the sites:
+//   * the coefficients of the chunk maps Y_t = b_t + c_t Y_{t-1} do not change in time, so every
+//     product of them that the scan needs is computed once per instance (registers) and a scan level
+//     is one complex multiply-add;
+//   * the carry into a warp is sum_k W_k b_{g-1-k} over the earlier warps' totals with constant
+//     weights W_k = prod c, cut where |W_k| < 1e-40 (FP64) or 1e-36 (float-float): with dx = 0.1 and
+//     dt = 0.25 the solve decays by 0.77 per site and a warp of 4-site chunks needs 3 terms;
+//   * each sweep is repeated from its exact carry instead of being corrected with chunk products
+//     (F, G of the CN tables): the same operation count, and no tables that depend on the chunking.
+// Warp totals travel as remote shared-memory stores to every later (forward) or earlier (backward)
+// CTA, each followed by a cluster barrier; a third barrier ends the step with the edge values of psi.
+// The observables' warp sums collect in rank 0 for 8 steps and are then summed by all its threads.
+//
+// Bound by the FP64 pipe of the cluster's SMs (FP64: 40 operations per site and about 100 per thread
+// and step, one warp per sub-partition) or by the latency of the scans (float-float); per step, one
+// CTA -> cluster: one 8001-site instance 108.8 -> 11.6 us in FP64 and 35.1 -> 5.4 us in float-float
+// (NC = 16), 601 sites 24.3 -> 6.7 us (FP64, NC = 8), 24 float-float instances 35.3 -> 8.8 us.
+#include <cooperative_groups.h>
+#include <cuda_runtime.h>
+
+#include "../../include/mma_tdse.h"
+#include "common.cuh"
+#include "df64.cuh"
+#include "tdse_host.cuh"
+#include "tdse_step.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace mma {
+namespace clk {
+
+constexpr int kT = 128, kW = kT / 32;  // one warp per sub-partition: FP64 issue is the limit, not latency
+constexpr int kMaxNC = 16;  // the largest cluster the hardware takes (over 8: opt-in)
+constexpr int kPhA = 8, kPhB = 4;  // lane = 4 a + b: e^{i F dt (4 a m dx)}, e^{i F dt (b m dx)}
+constexpr int kPh = kPhA + kPhB + kW + 1;  // + the warps' start phases + e^{-i F dt dx}
+constexpr int kPhSteps = kT / kPh;         // steps whose phases one pass of the CTA computes
+constexpr int kRing = 8, kObs = 5;         // steps of observables collected before they are summed
+constexpr int kGroups = 3;                 // thread groups that share those sums (kGroups kRing kObs <= kT)
+
+struct Args {
+    const mma_tdse_instance* insts;
+    int n_inst;
+    const mma_tdse_grid* grids;
+    const double* fields;
+    double* outputs;
+    double* psi_final;
+    double* snapshots;
+    int* counter;
+    int m_cap;      // sites per thread the shared memory was sized for
+    int64_t max_L;  // widest grid of the launch (padded sites), as the caller stated it
+};
+
+// ------------------------------------------------------------------ arithmetic of the two forms
+struct Fp64 {
+    typedef cd C;
+    typedef double R;  // a partial sum
+    static constexpr bool kFp64 = true;
+    static __device__ const C* table(const mma_tdse_grid& G) { return reinterpret_cast<const C*>(G.cn_tab); }
+    static __device__ C zero() { return cd{0.0, 0.0}; }
+    static __device__ C one() { return cd{1.0, 0.0}; }
+    static __device__ C neg(C a) { return cd{-a.re, -a.im}; }
+    static __device__ C conj(C a) { return cd{a.re, -a.im}; }
+    static __device__ bool tiny(C a) { return fabs(a.re) + fabs(a.im) < 1e-40; }
+    static __device__ C mul(C a, C b) { return cmul(a, b); }
+    static __device__ C fma(C a, C b, C z) { return cfma(a, b, z); }
+    static __device__ C fms(C a, C b, C z) { return cfms(a, b, z); }
+    static __device__ C rhs(C ib, C p, C a, C b)
+    {
+        return cmul(ib, cd{::fma(10.0, p.re, a.re + b.re), ::fma(10.0, p.im, a.im + b.im)});
+    }
+    static __device__ C update(C ph, C u, C p) { return cmul(ph, u - p); }
+    static __device__ C shup(C v, int d) { return cd{shfl_up(v.re, d), shfl_up(v.im, d)}; }
+    static __device__ C shdn(C v, int d) { return cd{shfl_down(v.re, d), shfl_down(v.im, d)}; }
+    static __device__ C bcast(C v, int l) { return cd{shfl_idx(v.re, l), shfl_idx(v.im, l)}; }
+    static __device__ C from(double re, double im) { return cd{re, im}; }
+    static __device__ void to_d(C v, double& re, double& im) { re = v.re, im = v.im; }
+    static __device__ R re(C v) { return v.re; }
+    static __device__ bool has_im(C v) { return v.im != 0.0; }
+    static __device__ R rzero() { return 0.0; }
+    static __device__ R radd(R a, R b) { return a + b; }
+    static __device__ R rxor(R a, int d) { return shfl_xor(a, d); }
+    static __device__ double rd(R a) { return a; }
+    struct Acc {
+        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0, w = 0.0;
+        __device__ void add(C pn, C gx, R p0, bool in)
+        {
+            const double n2 = ::fma(pn.re, pn.re, pn.im * pn.im);
+            a0 = ::fma(n2, gx.re, a0);
+            a1 = ::fma(n2, gx.im, a1);
+            a2 = ::fma(pn.re, p0, a2);
+            a3 = ::fma(pn.im, p0, a3);
+            if (in) w += n2;
+        }
+        // the imaginary part of a complex ground state: <psi0|psi> += conj(i p0i) psi
+        __device__ void add_im(C pn, R p0i)
+        {
+            a2 = ::fma(pn.im, p0i, a2);
+            a3 = ::fma(-pn.re, p0i, a3);
+        }
+        __device__ void get(R (&v)[4]) { v[0] = a0, v[1] = a1, v[2] = a2, v[3] = a3; }
+        __device__ R window() { return w; }
+    };
+};
+
+struct Df64 {
+    typedef dfk::pk C;
+    typedef dfk::df R;
+    static constexpr bool kFp64 = false;
+    static __device__ const C* table(const mma_tdse_grid& G) { return reinterpret_cast<const C*>(G.df_tab); }
+    static __device__ C zero() { return C{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
+    static __device__ C one() { return C{make_float2(1.f, 0.f), make_float2(0.f, 0.f)}; }
+    static __device__ C neg(C a) { return C{dfk::ng2(a.h), dfk::ng2(a.l)}; }
+    static __device__ C conj(C a) { return C{make_float2(a.h.x, -a.h.y), make_float2(a.l.x, -a.l.y)}; }
+    static __device__ bool tiny(C a) { return fabsf(a.h.x) + fabsf(a.h.y) < 1e-36f; }
+    static __device__ C mul(C a, C b) { return dfk::cmul_p(a, b); }
+    static __device__ C fma(C a, C b, C z) { return dfk::cfma_p(a, b, z); }
+    static __device__ C fms(C a, C b, C z) { return dfk::cfms_p(a, b, z); }
+    static __device__ C rhs(C ib, C p, C a, C b) { return dfk::cmul_pu(ib, dfk::ten_sum_p(p, a, b)); }
+    static __device__ C update(C ph, C u, C p)
+    {
+        float2 s, t;
+        dfk::two_sum2(u.h, dfk::ng2(p.h), s, t);
+        return dfk::cmul_p(ph, C{s, dfk::add2(t, dfk::sub2(u.l, p.l))});
+    }
+    static __device__ C shup(C v, int d) { return dfk::pshup(v, d); }
+    static __device__ C shdn(C v, int d) { return dfk::pshdn(v, d); }
+    static __device__ C bcast(C v, int l)
+    {
+        return C{make_float2(__shfl_sync(0xffffffffu, v.h.x, l), __shfl_sync(0xffffffffu, v.h.y, l)),
+                 make_float2(__shfl_sync(0xffffffffu, v.l.x, l), __shfl_sync(0xffffffffu, v.l.y, l))};
+    }
+    static __device__ C from(double re, double im)
+    {
+        const dfk::df a = dfk::from_d(re), b = dfk::from_d(im);
+        return C{make_float2(a.hi, b.hi), make_float2(a.lo, b.lo)};
+    }
+    static __device__ void to_d(C v, double& re, double& im)
+    {
+        re = (double)v.h.x + (double)v.l.x;
+        im = (double)v.h.y + (double)v.l.y;
+    }
+    static __device__ R re(C v) { return R{v.h.x, v.l.x}; }
+    static __device__ bool has_im(C v) { return v.h.y != 0.f; }
+    static __device__ R rzero() { return R{0.f, 0.f}; }
+    static __device__ R radd(R a, R b) { return dfk::add(a, b); }
+    static __device__ R rxor(R a, int d) { return dfk::shfl_xor_df(a, d); }
+    static __device__ double rd(R a) { return dfk::to_d(a); }
+    struct Acc {
+        C a01 = zero(), a23 = zero();
+        R w = rzero();
+        __device__ void add(C pn, C gx, R p0, bool in)
+        {
+            const R n2 = dfk::norm2_u(pn);
+            dfk::acc_mul_p(a01, n2.hi, n2.lo, gx);
+            dfk::acc_mul_p(a23, p0.hi, p0.lo, pn);
+            if (in) w = dfk::add(w, dfk::renorm(n2.hi, n2.lo));
+        }
+        __device__ void add_im(C pn, R p0i) { dfk::acc_mul_p(a23, p0i.hi, p0i.lo, C{dfk::mipair(pn.h), dfk::mipair(pn.l)}); }
+        __device__ void get(R (&v)[4])
+        {
+            const C x = dfk::renorm2(a01.h, a01.l), y = dfk::renorm2(a23.h, a23.l);
+            v[0] = R{x.h.x, x.l.x}, v[1] = R{x.h.y, x.l.y}, v[2] = R{y.h.x, y.l.x}, v[3] = R{y.h.y, y.l.y};
+        }
+        __device__ R window() { return w; }
+    };
+};
+
+// Dynamic shared memory: per padded site psi, sweep, 1/(6 beta), h, g, (-V', x) [16 bytes each] and
+// Re psi0 [8 bytes]; then the warp totals, their weights, the phases and the observables' ring.
+__host__ __device__ inline size_t site_bytes() { return 6 * 16 + 8; }
+__host__ __device__ inline size_t fixed_bytes(int nc)
+{
+    const size_t nw = (size_t)nc * kW;
+    return 16 * (2 * nw + 2 * kW * nw + 2 * kPhSteps * kPh) + 8 * (kRing * nw * kObs + kGroups * kRing * kObs);
+}
+
+template <class N>
+__global__ void __launch_bounds__(kT, 1) propagate_cluster_kernel(Args P)
+{
+    typedef typename N::C C;
+    typedef typename N::R R;
+    static_assert(sizeof(C) == 16 && sizeof(R) == 8, "shared-memory layout");
+    cg::cluster_group cluster = cg::this_cluster();
+    const int NC = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), NW = NC * kW;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, g = rank * kW + w;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int ML = P.m_cap * kT;
+    C* const psi = reinterpret_cast<C*>(smem);
+    C *const yv = psi + ML, *const ib = yv + ML, *const hh = ib + ML, *const gg = hh + ML, *const gx = gg + ML;
+    C *const totF = gx + ML, *const totB = totF + NW, *const wtF = totB + NW, *const wtB = wtF + kW * NW,
+             *const phs = wtB + kW * NW;
+    R* const p0 = reinterpret_cast<R*>(phs + 2 * kPhSteps * kPh);
+    R* const ring = p0 + ML;
+    R* const part = ring + kRing * NW * kObs;
+    __shared__ C edge[2];
+    __shared__ int s_inst;
+    __shared__ long long s_gate;
+    __shared__ int s_lo, s_hi;
+    __shared__ double s_red[kW];
+
+    for (;;) {
+        cluster.sync();  // no CTA still reads or writes the previous instance's state
+        if (rank == 0 && t == 0) {
+            const int v = atomicAdd(P.counter, 1);
+            for (int r = 0; r < NC; r++) *cluster.map_shared_rank(&s_inst, r) = v;
+        }
+        cluster.sync();
+        const int inst = s_inst;
+        if (inst >= P.n_inst) break;
+        const mma_tdse_instance I = P.insts[inst];
+        const mma_tdse_grid G = P.grids[I.grid];
+        const int64_t S = I.n_steps;
+        const int n = (int)G.n, m256 = (int)G.m;
+        const int64_t L = G.m * kThreads;
+        const double* f = P.fields + I.field_off;
+        double* out = P.outputs + I.out_off;
+        double *o_t = out, *o_e = out + (S + 1), *o_src = out + 2 * (S + 1), *o_ptot = out + 3 * (S + 1),
+               *o_pint = out + 4 * (S + 1), *o_x = out + 5 * (S + 1);
+        const double dt = G.dt, dx = G.dx;
+        const int m = (n + NC * kT - 1) / (NC * kT);
+        if (L > P.max_L || m > P.m_cap) {
+            // a grid wider than the launch was sized for: NaN outputs, as in the one-CTA kernel
+            for (int64_t e = (int64_t)rank * kT + t; e < 6 * (S + 1); e += NC * kT)
+                out[e] = __longlong_as_double(0x7ff8000000000000LL);
+            continue;
+        }
+        const int c0 = rank * kT + t;  // chunk of this thread: sites c0 m .. c0 m + m - 1
+        const int s0 = c0 * m;
+        // ---- tables of the thread's sites (the grid's tables are interleaved for 256 chunks of m256)
+        const C* tab = N::table(G);
+        C cF = N::one(), cB = N::one();
+        bool im = false;
+        for (int i = 0; i < m; i++) {
+            const int j = s0 + i, q = i * kT + t;
+            C a = N::zero(), h = a, gq = a, x = a, p = a;
+            if (j < n) {
+                const int64_t e = (int64_t)(j % m256) * kThreads + j / m256;
+                a = tab[CN_IB6 * L + e];
+                h = tab[CN_H * L + e];
+                gq = tab[CN_G * L + e];
+                x = tab[CN_GVX * L + e];
+                p = tab[CN_PSI0 * L + e];
+            }
+            ib[q] = a;
+            hh[q] = h;
+            gg[q] = gq;
+            gx[q] = x;
+            psi[q] = p;
+            p0[q] = N::re(p);
+            im |= N::has_im(p);
+            cF = N::mul(cF, N::neg(h));
+            cB = N::mul(cB, N::neg(gq));
+        }
+        // ---- zero gate (prop.c:125-134) and population window (tools_algorithmic.c:19-43)
+        if (t == 0) {
+            s_gate = S;
+            s_lo = s_hi = n - 1;
+            edge[0] = edge[1] = N::zero();
+        }
+        const bool psi0_im = __syncthreads_or(im);
+        for (int64_t b = 0; b < S; b += kT) {
+            const int64_t k = b + t;
+            bool hit = false;
+            if (k < S) {
+                double fa = (k < I.n_field) ? f[k] : 0.0, fb = (k + 1 < I.n_field) ? f[k + 1] : 0.0;
+                if (fabs(fa) <= I.gate_floor) fa = 0.0;
+                if (fabs(fb) <= I.gate_floor) fb = 0.0;
+                hit = fa * fb <= 0.0;
+                if (hit) atomicMin(&s_gate, (long long)k);
+            }
+            if (__syncthreads_or(hit)) break;
+        }
+        // lo: the first i with -x_int <= x[i+1] (0 where the window starts left of the grid); hi: one
+        // past the first i with x_int <= x[i+1]; both within the grid
+        const double x0 = G.x[0];
+        for (int i = t; i + 1 < n; i += kT) {
+            const double xn = G.x[i + 1];
+            if (-G.x_int <= xn) atomicMin(&s_lo, i);
+            if (G.x_int <= xn) atomicMin(&s_hi, i + 1);
+            if (-G.x_int <= xn && G.x_int <= xn) break;
+        }
+        __syncthreads();
+        const int lo = (-G.x_int < x0) ? 0 : s_lo, hi = (G.x_int < x0) ? 0 : s_hi;
+        const int64_t gate = s_gate;
+        const bool warp_win = __any_sync(0xffffffffu, s0 <= hi && s0 + m > lo);
+        auto applied = [&](int64_t k) { return (k <= gate || k >= I.n_field || k >= S) ? 0.0 : f[k]; };
+
+        // ---- constants of the scans: products of the chunk coefficients over 1, 2, 4, 8, 16 chunks
+        C f_lv[5], b_lv[5];
+#pragma unroll
+        for (int l = 0; l < 5; l++) {
+            f_lv[l] = cF;
+            b_lv[l] = cB;
+            const C up = N::shup(cF, 1 << l), dn = N::shdn(cB, 1 << l);
+            if (lane >= (1 << l)) cF = N::mul(cF, up);
+            if (lane + (1 << l) < 32) cB = N::mul(cB, dn);
+        }
+        const C wF = N::bcast(cF, 31), wB = N::bcast(cB, 0);
+        const C f_ex = N::shup(cF, 1), b_ex = N::shdn(cB, 1);  // products of the chunks before (after) this one
+        if (lane < NC) {
+            cluster.map_shared_rank(totF, lane)[g] = wF;
+            cluster.map_shared_rank(totB, lane)[g] = wB;
+        }
+        cluster.sync();
+        int KF = 0, KB = 0;
+        if (lane == 0) {
+            C W = N::one();
+            for (; KF < g && !N::tiny(W); KF++) {
+                wtF[w * NW + KF] = W;
+                W = N::mul(W, totF[g - 1 - KF]);
+            }
+            W = N::one();
+            for (; KB < NW - 1 - g && !N::tiny(W); KB++) {
+                wtB[w * NW + KB] = W;
+                W = N::mul(W, totB[g + 1 + KB]);
+            }
+        }
+        KF = __shfl_sync(0xffffffffu, KF, 0);
+        KB = __shfl_sync(0xffffffffu, KB, 0);
+        auto send_edges = [&] {
+            if (t == 0 && rank > 0) *cluster.map_shared_rank(&edge[1], rank - 1) = psi[0];
+            if (t == kT - 1 && rank + 1 < NC) *cluster.map_shared_rank(&edge[0], rank + 1) = psi[(m - 1) * kT + t];
+        };
+        send_edges();
+        if (rank == 0) {  // initial window population (prop.c:87-93)
+            double v = 0.0;
+            for (int j = lo + t; j <= hi; j += kT)
+                v += G.psi0[2 * j] * G.psi0[2 * j] + G.psi0[2 * j + 1] * G.psi0[2 * j + 1];
+#pragma unroll
+            for (int d = 16; d >= 1; d >>= 1) v += shfl_xor(v, d);
+            if (lane == 0) s_red[w] = v;
+            __syncthreads();
+            if (t == 0) {
+                o_t[0] = I.tmin;
+                o_e[0] = 0.0;
+                o_src[0] = 0.0;
+                o_ptot[0] = 1.0;
+                o_x[0] = 0.0;
+                o_pint[0] = (s_red[0] + s_red[1]) + (s_red[2] + s_red[3]);
+            }
+        }
+        double tt = I.tmin;
+        // rank 0: the series of steps k0 .. k0 + cnt - 1 from the ring (prop.c:293-347)
+        auto flush = [&](int64_t k0, int cnt) {
+            const int grp = t / (kRing * kObs), v = t % (kRing * kObs);
+            if (grp < kGroups) {
+                R s = N::rzero();
+                for (int q = grp; q < NW; q += kGroups) s = N::radd(s, ring[((v / kObs) * NW + q) * kObs + v % kObs]);
+                part[grp * kRing * kObs + v] = s;
+            }
+            __syncthreads();
+            const int c = t % kObs;
+            if (t < cnt * kObs) {
+                auto total = [&](int q) {
+                    R s = part[q];
+#pragma unroll
+                    for (int r = 1; r < kGroups; r++) s = N::radd(s, part[r * kRing * kObs + q]);
+                    return N::rd(s);
+                };
+                const int64_t k = k0 + t / kObs;
+                const double v0 = total(t);
+                if (c == 0) {
+                    const double F = applied(k);
+                    o_e[k + 1] = F;
+                    o_src[k + 1] = -v0 + F;
+                } else if (c == 1) {
+                    o_x[k + 1] = v0;
+                } else if (c == 2) {
+                    const double v1 = total(t + 1);
+                    o_ptot[k + 1] = v0 * v0 + v1 * v1;
+                } else if (c == 4) {
+                    o_pint[k + 1] = v0;
+                }
+            }
+            if (t == kT - 1)
+                for (int s = 0; s < cnt; s++) {  // t accumulates by repeated addition, as the reference's
+                    tt += dt;
+                    o_t[k0 + s + 1] = tt;
+                }
+            __syncthreads();  // part is rewritten by the next flush
+        };
+        const bool ckpt = I.ckpt_every > 0 && I.ckpt_off >= 0 && P.snapshots;
+        auto store_state = [&](double* dst) {  // natural order, 2 doubles per site
+            for (int i = 0; i < m; i++)
+                if (s0 + i < n) {
+                    double re, imv;
+                    N::to_d(psi[i * kT + t], re, imv);
+                    st2(dst + 2 * (s0 + i), cd{re, imv});
+                }
+        };
+        if (ckpt) store_state(P.snapshots + I.ckpt_off);
+        // the phases of kPhSteps steps from k0 on, one angle per thread, into the half of the table that
+        // no thread reads: a batch is computed during the last step of the one before, so the barriers
+        // of that step separate it from its readers
+        auto phases = [&](int64_t k0) {
+            if (t >= kPhSteps * kPh) return;
+            const int a = t % kPh;
+            const double Fdt = applied(k0 + t / kPh) * dt, step = (double)m * dx;
+            double ang;
+            if (a < kPhA) ang = Fdt * (step * (4 * a));
+            else if (a < kPhA + kPhB) ang = Fdt * (step * (a - kPhA));
+            else if (a < kPh - 1)  // the last site of the warp's first chunk
+                ang = Fdt * (x0 + dx * (double)((rank * kT + 32 * (a - kPhA - kPhB)) * m + m - 1));
+            else ang = -(Fdt * dx);
+            double sn, cs;
+            sincos(ang, &sn, &cs);
+            phs[(int)(k0 / kPhSteps % 2) * kPhSteps * kPh + t] = N::from(cs, sn);
+        };
+        phases(0);
+        cluster.sync();  // weights computed from totF / totB, edges in place
+
+        for (int64_t k = 0; k < S; k++) {
+            // ---- forward sweep from zero of the right-hand side 2 M2 psi: the chunk's end value
+            C pm = (t == 0) ? edge[0] : psi[(m - 1) * kT + t - 1];
+            const C nx = (t == kT - 1) ? edge[1] : psi[t + 1];
+            C pc = psi[t];
+            C b = N::zero();
+#pragma unroll 2
+            for (int i = 0; i < m; i++) {
+                const int q = i * kT + t;
+                const C pn = (i + 1 < m) ? psi[q + kT] : nx;
+                const C r = N::rhs(ib[q], pc, pm, pn);
+                yv[q] = r;
+                b = N::fms(hh[q], b, r);
+                pm = pc;
+                pc = pn;
+            }
+#pragma unroll
+            for (int l = 0; l < 5; l++) {
+                const C up = N::shup(b, 1 << l);
+                if (lane >= (1 << l)) b = N::fma(f_lv[l], up, b);
+            }
+            C tot = N::bcast(b, 31);
+            if (lane >= rank && lane < NC) cluster.map_shared_rank(totF, lane)[g] = tot;
+            cluster.barrier_arrive();
+            const int kp = (int)(k % kPhSteps);
+            if (kp == kPhSteps - 1) phases(k + 1);
+            C bx = N::shup(b, 1);
+            cluster.barrier_wait();
+            if (rank == 0 && k > 0 && k % kRing == 0) flush(k - kRing, kRing);
+            C yw = N::zero();
+            for (int q = 0; q < KF; q++) yw = N::fma(wtF[w * NW + q], totF[g - 1 - q], yw);
+            // ---- forward sweep from the exact carry, backward sweep from zero
+            C y = lane == 0 ? yw : N::fma(f_ex, yw, bx);
+#pragma unroll 2
+            for (int i = 0; i < m; i++) {
+                const int q = i * kT + t;
+                y = N::fms(hh[q], y, yv[q]);
+                yv[q] = y;
+            }
+            b = y;
+#pragma unroll 2
+            for (int i = m - 2; i >= 0; i--) {
+                const int q = i * kT + t;
+                b = N::fms(gg[q], b, yv[q]);
+            }
+#pragma unroll
+            for (int l = 0; l < 5; l++) {
+                const C dn = N::shdn(b, 1 << l);
+                if (lane + (1 << l) < 32) b = N::fma(b_lv[l], dn, b);
+            }
+            tot = N::bcast(b, 0);
+            if (lane <= rank) cluster.map_shared_rank(totB, lane)[g] = tot;
+            cluster.barrier_arrive();
+            bx = N::shdn(b, 1);
+            const C* ps = phs + ((int)(k / kPhSteps % 2) * kPhSteps + kp) * kPh;
+            C ph = N::mul(N::mul(ps[lane >> 2], ps[kPhA + (lane & 3)]), ps[kPhA + kPhB + w]);
+            const C zc = ps[kPh - 1];
+            cluster.barrier_wait();
+            C uw = N::zero();
+            for (int q = 0; q < KB; q++) uw = N::fma(wtB[w * NW + q], totB[g + 1 + q], uw);
+            // ---- backward sweep from the exact carry, CN update, phase e^{+i F dt x}, observables
+            C u = lane == 31 ? uw : N::fma(b_ex, uw, bx);
+            typename N::Acc acc;
+#pragma unroll 2
+            for (int i = m - 1; i >= 0; i--) {
+                const int q = i * kT + t, j = s0 + i;
+                u = N::fms(gg[q], u, yv[q]);
+                const C pn = N::update(ph, u, psi[q]);
+                psi[q] = pn;
+                ph = N::mul(ph, zc);
+                acc.add(pn, gx[q], p0[q], j >= lo && j <= hi);
+                if (psi0_im && j < n) {
+                    const int64_t e = (int64_t)(j % m256) * kThreads + j / m256;
+                    acc.add_im(pn, N::re(N::mul(C(N::from(0.0, -1.0)), tab[CN_PSI0 * L + e])));
+                }
+            }
+            send_edges();
+            cluster.barrier_arrive();
+            {   // warp sums: four values in six additions (each level halves what a lane carries)
+                R v[4];
+                acc.get(v);
+                const bool h16 = lane & 16, h8 = lane & 8;
+                R a = N::radd(h16 ? v[2] : v[0], N::rxor(h16 ? v[0] : v[2], 16));
+                R c = N::radd(h16 ? v[3] : v[1], N::rxor(h16 ? v[1] : v[3], 16));
+                R s = N::radd(h8 ? c : a, N::rxor(h8 ? a : c, 8));
+#pragma unroll
+                for (int d = 4; d >= 1; d >>= 1) s = N::radd(s, N::rxor(s, d));
+                R win = N::rzero();
+                if (warp_win) {
+                    win = acc.window();
+#pragma unroll
+                    for (int d = 16; d >= 1; d >>= 1) win = N::radd(win, N::rxor(win, d));
+                }
+                R* dst = cluster.map_shared_rank(ring, 0) + ((int)(k % kRing) * NW + g) * kObs;
+                if ((lane & 7) == 0) dst[lane >> 3] = s;
+                if (lane == 1) dst[4] = win;
+            }
+            if (ckpt && (k + 1) % I.ckpt_every == 0 && k + 1 < S)
+                store_state(P.snapshots + I.ckpt_off + (k + 1) / I.ckpt_every * 2 * (int64_t)n);
+            if (I.snap_off >= 0 && P.snapshots) {  // prop.c:248-263
+                int64_t slot = -1;
+                if (k % I.snap_every == 0 && k / I.snap_every < I.n_snap - 1) slot = k / I.snap_every;
+                if (k == S - 1) slot = I.n_snap - 1;
+                if (slot >= 0) store_state(P.snapshots + I.snap_off + slot * 2 * (int64_t)n);
+            }
+            cluster.barrier_wait();
+        }
+        cluster.sync();  // the last steps' sums are in rank 0's ring
+        if (rank == 0) flush((S - 1) / kRing * kRing, (int)(S - (S - 1) / kRing * kRing));
+        if (P.psi_final && I.psi_off >= 0) store_state(P.psi_final + I.psi_off);
+    }
+}
+
+}  // namespace clk
+}  // namespace mma
+
+using namespace mma;
+
+namespace {
+
+template <class N>
+int launch(const clk::Args& A, int nc, int clusters, size_t smem, cudaStream_t st)
+{
+    auto k = clk::propagate_cluster_kernel<N>;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        return MMA_ERR_CUDA;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(clusters * nc));
+    cfg.blockDim = dim3(clk::kT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)nc;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, A) == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+}
+
+template <class N>
+int active_clusters(int nc, size_t smem)
+{
+    auto k = clk::propagate_cluster_kernel<N>;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)nc);
+    cfg.blockDim = dim3(clk::kT);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)nc;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int c = 0;
+    if (cudaOccupancyMaxActiveClusters(&c, k, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return c;
+}
+
+}  // namespace
+
+namespace mma {
+
+// Where the line lies between one CTA and a cluster per instance, and the cluster size: the smallest
+// expected time of a step of the whole batch.  The models were fitted to runs of 1 to 304 instances on
+// grids of 601 to 8001 sites (us per step, measured / model):
+//   one CTA    FP64   601 sites  24.3 / 24.3    8001 sites  108.8 / 108.7   256 x 4001 sites  125 / 124
+//              df64   601 sites   7.8 /  7.8    8001 sites   35.1 /  35.1   304 x 8001 sites  58.8 / 58.9
+//   cluster    FP64  8001 sites  NC = 4  29.0 / 28.9   8  17.3 / 17.3   16  11.7 / 11.5;  256 x 4001, NC = 2  115 / 116
+//              df64  8001 sites  NC = 4  10.1 / 10.1   8   6.9 /  7.2   16   5.6 /  5.7
+// FP64 is bound by the FP64 pipe, so CTAs that share an SM add their times (all but the barriers'); the
+// float-float form by latency, so a second CTA costs about two thirds of the first.
+namespace {
+double one_cta_us(int m256, int precision, int n_inst, int sms)
+{
+    if (precision != 2) return (double)((n_inst + sms - 1) / sms) * (15.6 + 2.91 * m256);
+    const double one = 5.0 + 0.94 * m256, two = 8.3 + 1.58 * m256;
+    const int full = n_inst / (2 * sms), rest = n_inst % (2 * sms);
+    return full * two + (rest == 0 ? 0.0 : rest <= sms ? one : two);
+}
+double cluster_us(int m, int precision, int waves, int per_sm)
+{
+    if (precision != 2) return waves * (2.4 + per_sm * (3.3 + 1.45 * m));
+    return waves * (4.2 + 0.37 * m) * (1.0 + 0.65 * (per_sm - 1));
+}
+}  // namespace
+
+bool choose_cluster(int max_m, int precision, int n_inst, int sms, ClusterPlan* plan)
+{
+    double best = one_cta_us(max_m, precision, n_inst, sms);
+    bool found = false, tried[clk::kMaxNC + 1] = {};
+    for (;;) {
+        // the most promising size not looked at yet, if every SM could be filled: the number of
+        // clusters that are really resident depends on the GPU's partition and is asked for it alone
+        int pick = 0;
+        double promise = best;
+        ClusterPlan cand{};
+        for (int nc = 1; nc <= clk::kMaxNC; nc++) {
+            if (tried[nc]) continue;
+            const int m = (max_m * kThreads + nc * clk::kT - 1) / (nc * clk::kT);
+            const size_t smem = (size_t)m * clk::kT * clk::site_bytes() + clk::fixed_bytes(nc);
+            if (smem > 226 * 1024 || (nc > 1 && (nc - 1) * m * clk::kT >= max_m * kThreads)) continue;
+            const int fit = sms * (smem > 112 * 1024 ? 1 : 2) / nc;
+            const int run = fit < n_inst ? fit : n_inst;
+            const double us = run < 1 ? best : cluster_us(m, precision, (n_inst + run - 1) / run, (run * nc + sms - 1) / sms);
+            if (us < promise) {
+                promise = us;
+                pick = nc;
+                cand = ClusterPlan{nc, m, smem, 0};
+            }
+        }
+        if (!pick) return found;
+        tried[pick] = true;
+        cand.active = precision == 2 ? active_clusters<clk::Df64>(pick, cand.smem) : active_clusters<clk::Fp64>(pick, cand.smem);
+        if (cand.active < 1) continue;
+        const int run = cand.active < n_inst ? cand.active : n_inst;
+        const double us = cluster_us(cand.m, precision, (n_inst + run - 1) / run, (run * pick + sms - 1) / sms);
+        if (us < best) {
+            best = us;
+            *plan = cand;
+            found = true;
+        }
+    }
+}
+
+int launch_cluster(const ClusterPlan& p, const mma_tdse_instance* insts, int n_inst, const mma_tdse_grid* grids,
+                   const mma_tdse_buffers* bufs, int max_m, int precision, void* stream)
+{
+    cudaStream_t st = (cudaStream_t)stream;
+    if (cudaMemsetAsync(bufs->counter, 0, sizeof(int), st) != cudaSuccess) return MMA_ERR_CUDA;
+    clk::Args A{insts, n_inst, grids, bufs->fields, bufs->outputs, bufs->psi_final, bufs->snapshots, bufs->counter,
+                p.m, (int64_t)max_m * kThreads};
+    const int clusters = p.active < n_inst ? p.active : n_inst;
+    return precision == 2 ? launch<clk::Df64>(A, p.nc, clusters, p.smem, st)
+                          : launch<clk::Fp64>(A, p.nc, clusters, p.smem, st);
+}
+
+}  // namespace mma

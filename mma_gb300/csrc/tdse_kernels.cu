@@ -18,6 +18,7 @@
 
 #include "../../include/mma_tdse.h"
 #include "common.cuh"
+#include "tdse_host.cuh"
 #include "tdse_solver.cuh"
 #include "tdse_step.cuh"
 
@@ -575,12 +576,17 @@ extern "C" int mma_tdse_propagate_ex(const mma_tdse_instance* insts, int n_inst,
         grid_ctas = precision == 1 ? mma_tdse_c64_default_ctas(max_m, cta_threads) : mma_tdse_default_ctas(max_m, precision);
     if (grid_ctas <= 0) return MMA_ERR_TOO_LARGE;  // no complex64 kernel for this shape
     if (grid_ctas > n_inst) grid_ctas = n_inst;
+    // a caller that asks for fewer CTAs than the batch could use keeps the one-CTA kernels and that limit
+    const bool limited = precision != 1 && grid_ctas < n_inst && grid_ctas < mma_tdse_default_ctas(max_m, precision);
     if (precision == 1) {
         // max_m is the common m32 of the batch's complex64 tables, cta_threads their CTA size
         return mma_tdse_propagate_c64_impl(insts, n_inst, grids, bufs, max_m, cta_threads, grid_ctas, stream);
     }
     if (cta_threads != 0 && cta_threads != kThreads) return MMA_ERR_UNSUPPORTED;
     if (bufs->scratch_bytes < mma_tdse_scratch_bytes(max_m, grid_ctas, precision)) return MMA_ERR_ARG;
+    ClusterPlan cp;  // instances spread over clusters where the batch leaves SMs idle (tdse_cluster.cu)
+    if (!limited && choose_cluster(max_m, precision, n_inst, sm_count(), &cp))
+        return launch_cluster(cp, insts, n_inst, grids, bufs, max_m, precision, stream);
     if (precision == 2)  // float-float form: the FP64 layout, psi in scratch, two CTAs per SM
         return mma_tdse_propagate_df64_impl(insts, n_inst, grids, bufs, max_m, grid_ctas, stream);
     cudaStream_t st = (cudaStream_t)stream;
