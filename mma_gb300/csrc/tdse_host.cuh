@@ -22,4 +22,7 @@ bool choose_cluster(int max_m, int precision, int n_inst, int sms, ClusterPlan* 
 int launch_cluster(const ClusterPlan& p, const mma_tdse_instance* insts, int n_inst, const mma_tdse_grid* grids,
                    const mma_tdse_buffers* bufs, int max_m, int precision, void* stream);
 
+// x and the ground state of one grid, without its Crank-Nicolson tables (tdse_kernels.cu)
+int ground_state_only(const mma_tdse_grid* grid_dev, cudaStream_t st);
+
 }  // namespace mma

@@ -25,40 +25,114 @@
 namespace mma {
 
 // ------------------------------------------------------------------------------------------
-// Sequential factorisation of one tridiagonal matrix (thread 0), results chunk-interleaved.
+// Factorisation of one tridiagonal matrix by the whole CTA, results chunk-interleaved.
 // Row j: sub a_j (column j-1), diagonal b_j, super c_j (column j+1).
+//
+// The pivots beta_j = b_j - a_j c_{j-1} / beta_{j-1} are a chain of Moebius maps, beta = p/q with
+// (p, q) -> (b_j p - e_j q, p), e_j = a_j c_{j-1}.  Each thread multiplies the 2x2 matrices of its m
+// sites (rescaled by powers of two), a CTA scan composes them, and the thread then runs the plain
+// recurrence over its chunk from the pivot just before it.  One thread running the whole chain took
+// 10 ms for 8001 sites (dependent FP64 divisions), 18 ms with the complex matrix of the step; split
+// over 256 threads the two take 0.1 ms.
 // ------------------------------------------------------------------------------------------
-template <typename T, typename RowFn>
-__device__ void factorise(int64_t n, int64_t m, T* ib, T* h, T* g, double rhs_scale, RowFn row)
+template <typename T>
+struct Moebius {
+    T a, b, c, d;  // (p, q) -> (a p + b q, c p + d q)
+};
+__device__ __forceinline__ double mag_(double v) { return fabs(v); }
+__device__ __forceinline__ double mag_(cd v) { return fmax(fabs(v.re), fabs(v.im)); }
+__device__ __forceinline__ double scale_(double v, double s) { return v * s; }
+__device__ __forceinline__ cd scale_(cd v, double s) { return cd{v.re * s, v.im * s}; }
+__device__ __forceinline__ double neg_(double v) { return -v; }
+__device__ __forceinline__ cd neg_(cd v) { return cd{-v.re, -v.im}; }
+__device__ __forceinline__ double inv_(double v) { return 1.0 / v; }
+__device__ __forceinline__ cd inv_(cd v)
 {
-    T a, b, c, beta, ibeta;
-    row(0, a, b, c);
-    beta = b;
+    const double s = 1.0 / fma(v.re, v.re, v.im * v.im);
+    return cd{v.re * s, -v.im * s};
+}
+
+template <typename T>
+__device__ __forceinline__ void rescale(Moebius<T>& M)
+{
+    int e;
+    frexp(fmax(fmax(mag_(M.a), mag_(M.b)), fmax(mag_(M.c), mag_(M.d))), &e);
+    const double s = ldexp(1.0, -e);
+    M = Moebius<T>{scale_(M.a, s), scale_(M.b, s), scale_(M.c, s), scale_(M.d, s)};
+}
+
+// B after A
+template <typename T>
+__device__ __forceinline__ Moebius<T> compose(const Moebius<T>& B, const Moebius<T>& A)
+{
+    Moebius<T> M{axpy_(B.a, A.a, mul_(B.b, A.c)), axpy_(B.a, A.b, mul_(B.b, A.d)), axpy_(B.c, A.a, mul_(B.d, A.c)),
+                 axpy_(B.c, A.b, mul_(B.d, A.d))};
+    rescale(M);
+    return M;
+}
+
+// `warp`: kWarps entries of shared scratch.  Contains __syncthreads.
+template <typename T, typename RowFn>
+__device__ void factorise(int64_t n, int64_t m, T* ib, T* h, T* g, double rhs_scale, Moebius<T>* warp, RowFn row)
+{
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     T one;
     if constexpr (sizeof(T) == sizeof(double)) one = 1.0; else one = cd{1.0, 0.0};
-    for (int64_t j = 0; j < n; j++) {
-        T aj, bj, cj;
-        row(j, aj, bj, cj);
-        if (j > 0) {
-            // gamma_j = c_{j-1}/beta_{j-1} ; beta_j = b_j - a_j gamma_j
-            T gam;
-            if constexpr (sizeof(T) == sizeof(double)) gam = c / beta; else gam = cdiv(c, beta);
-            g[qidx(j - 1, m)] = gam;
-            if constexpr (sizeof(T) == sizeof(double)) beta = bj - aj * gam; else beta = bj - cmul(aj, gam);
-        }
-        if constexpr (sizeof(T) == sizeof(double)) {
-            ibeta = 1.0 / beta;
-            ib[qidx(j, m)] = ibeta * rhs_scale;
-            h[qidx(j, m)] = (j > 0) ? aj * ibeta : 0.0;
-        } else {
-            ibeta = cdiv(one, beta);
-            ib[qidx(j, m)] = cd{ibeta.re * rhs_scale, ibeta.im * rhs_scale};
-            h[qidx(j, m)] = (j > 0) ? cmul(aj, ibeta) : cd{0.0, 0.0};
-        }
-        c = cj;
-        a = aj;
+    const T zero = zero_(one);
+    const int64_t j0 = t * m, j1 = j0 + m < n ? j0 + m : n;
+    T a, b, c, cprev = zero;  // cprev: the super-diagonal of the row before
+    if (j0 > 0 && j0 < n) row(j0 - 1, a, b, cprev);
+    // the chunk's map; row 0 has no pivot before it: (p, q) -> (b_0 p, p)
+    Moebius<T> M{one, zero, zero, one};
+    T cp = cprev;
+    for (int64_t j = j0; j < j1; j++) {
+        row(j, a, b, c);
+        const T e = mul_(a, cp);  // a_0 = 0
+        M = Moebius<T>{axpy_(b, M.a, neg_(mul_(e, M.c))), axpy_(b, M.b, neg_(mul_(e, M.d))), M.a, M.b};
+        if (((j - j0) & 7) == 7) rescale(M);
+        cp = c;
     }
-    g[qidx(n - 1, m)] = T{};
+    rescale(M);
+#pragma unroll 1
+    for (int d = 1; d < 32; d <<= 1) {
+        const Moebius<T> up{shup_(M.a, d), shup_(M.b, d), shup_(M.c, d), shup_(M.d, d)};
+        if (lane >= d) M = compose(M, up);
+    }
+    if (lane == 31) warp[w] = M;
+    __syncthreads();
+    // the pivot before the chunk: the maps of the earlier warps, then those of the earlier lanes, on (1, 0)
+    T p = one, q = zero;
+    for (int v = 0; v < w; v++) {
+        const Moebius<T> W = warp[v];
+        const T pn = axpy_(W.a, p, mul_(W.b, q)), qn = axpy_(W.c, p, mul_(W.d, q));
+        int e;
+        frexp(fmax(mag_(pn), mag_(qn)), &e);
+        p = scale_(pn, ldexp(1.0, -e));
+        q = scale_(qn, ldexp(1.0, -e));
+    }
+    const Moebius<T> X{shup_(M.a, 1), shup_(M.b, 1), shup_(M.c, 1), shup_(M.d, 1)};
+    if (lane > 0) {
+        const T pn = axpy_(X.a, p, mul_(X.b, q)), qn = axpy_(X.c, p, mul_(X.d, q));
+        p = pn;
+        q = qn;
+    }
+    T ibeta = (j0 > 0 && j0 < n) ? mul_(q, inv_(p)) : zero;  // 1 / beta_{j0 - 1}
+    for (int64_t j = j0; j < j1; j++) {
+        row(j, a, b, c);
+        T beta = b;
+        if (j > 0) {
+            // gamma_{j-1} = c_{j-1} / beta_{j-1}; beta_j = b_j - a_j gamma_{j-1}
+            const T gam = mul_(cprev, ibeta);
+            g[qidx(j - 1, m)] = gam;
+            beta = axpy_(neg_(a), gam, b);
+        }
+        ibeta = inv_(beta);
+        ib[qidx(j, m)] = scale_(ibeta, rhs_scale);
+        h[qidx(j, m)] = (j > 0) ? mul_(a, ibeta) : zero;
+        cprev = c;
+    }
+    if (t == 0) g[qidx(n - 1, m)] = zero;
+    __syncthreads();
 }
 
 // Chunk products F (forward from the chunk start) and G (backward from the chunk end).
@@ -205,17 +279,20 @@ __device__ void ground_state(const mma_tdse_grid& G, const double* tab, double* 
 // ------------------------------------------------------------------------------------------
 // Grid builder.  mode 0: x, ground state, CN tables.  mode 1: CN tables from the grid's
 // existing x and psi0 (a caller-supplied ground state, as the legacy call1DTDSE allows).
+// mode 2 (library-internal): x and ground state only.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_grid* grids, int mode)
 {
     __shared__ double red[kWarps * 4];
     __shared__ double sc[2 * kWarps], sb[2 * kWarps];
+    __shared__ Moebius<cd> maps[kWarps];
+    Moebius<double>* const rmaps = reinterpret_cast<Moebius<double>*>(maps);
     const mma_tdse_grid G = grids[blockIdx.x];
     const int t = threadIdx.x;
     const int64_t n = G.n, m = G.m, L = m * kThreads, num_r = n - 1;
     const double dx = G.dx, a = G.trg_a, dt = G.dt;
 
-    if (mode == 0) {
+    if (mode != 1) {
         // separately rounded multiply and subtract, as the reference's x86 build evaluates
         // (double)k dx - xmax (no fused multiply-add)
         const double xmax = __dmul_rn(__dmul_rn(0.5, (double)num_r), dx);
@@ -226,12 +303,12 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
     for (int64_t j = t; j < n; j += kThreads) G.gv[j] = soft_coulomb(G.x[j], a);
     __syncthreads();
     const double* V = G.gv;
-    if (mode == 0) {
+    if (mode != 1) {
         // ground-state tables (tridiag.c:101-115)
         double* gtab = G.gs_tab;
         for (int64_t q = t; q < GS_SLOTS * L; q += kThreads) gtab[q] = 0.0;
         __syncthreads();
-        if (t == 0) {
+        {
             const double E = G.Eguess, k0 = -0.5 / (dx * dx), d0 = 1.0 / (dx * dx);
             auto row = [&](int64_t j, double& aj, double& bj, double& cj) {
                 const double vj = V[j];
@@ -239,14 +316,14 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
                 bj = 10.0 * vj / 12.0 + d0 - 10.0 * E / 12.0;
                 cj = (j + 1 < n) ? k0 - E / 12.0 + V[j + 1] / 12.0 : 0.0;
             };
-            factorise<double>(n, m, gtab + GS_IB12 * L, gtab + GS_H * L, gtab + GS_G * L, 1.0 / 12.0, row);
+            factorise<double>(n, m, gtab + GS_IB12 * L, gtab + GS_H * L, gtab + GS_G * L, 1.0 / 12.0, rmaps, row);
         }
-        __syncthreads();
         chunk_products<double>(m, gtab + GS_H * L, gtab + GS_G * L, gtab + GS_F * L, gtab + GS_GG * L);
         __syncthreads();
         // the CN table area doubles as the ground-state work space (3 L of 2*CN_SLOTS*L)
         double* work = G.cn_tab;
         ground_state(G, gtab, work, work + L, work + 2 * L, red, sc, sb, G.psi0);
+        if (mode == 2) return;
         __syncthreads();
     }
     // Crank-Nicolson tables (prop.c:138-159): row j sub (1/12, w_{j-1}), diag (10/12, d_j),
@@ -256,7 +333,7 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
     cd* ctab = reinterpret_cast<cd*>(G.cn_tab);
     for (int64_t q = t; q < CN_SLOTS * L; q += kThreads) ctab[q] = cd{0.0, 0.0};
     __syncthreads();
-    if (t == 0) {
+    {
         const double hdt = 0.5 * dt;
         auto row = [&](int64_t j, cd& aj, cd& bj, cd& cj) {
             const double vj = V[j];
@@ -264,9 +341,8 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
             bj = cd{10.0 / 12.0, hdt * (1.0 / (dx * dx)) + hdt * 10 / 12. * vj};
             cj = (j + 1 < n) ? cd{1.0 / 12.0, hdt * (-0.5 / (dx * dx)) + hdt * 1 / 12. * V[j + 1]} : cd{0.0, 0.0};
         };
-        factorise<cd>(n, m, ctab + CN_IB6 * L, ctab + CN_H * L, ctab + CN_G * L, 1.0 / 6.0, row);
+        factorise<cd>(n, m, ctab + CN_IB6 * L, ctab + CN_H * L, ctab + CN_G * L, 1.0 / 6.0, maps, row);
     }
-    __syncthreads();
     chunk_products<cd>(m, ctab + CN_H * L, ctab + CN_G * L, ctab + CN_F * L, ctab + CN_GG * L);
     __syncthreads();
     if (G.adj_tab) {
@@ -275,7 +351,7 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
         cd* atab = reinterpret_cast<cd*>(G.adj_tab);
         for (int64_t q = t; q < ADJ_SLOTS * L; q += kThreads) atab[q] = cd{0.0, 0.0};
         __syncthreads();
-        if (t == 0) {
+        {
             const double hdt = 0.5 * dt;
             auto row = [&](int64_t j, cd& aj, cd& bj, cd& cj) {
                 const double wj = hdt * (-0.5 / (dx * dx)) + hdt * 1 / 12. * V[j];
@@ -283,9 +359,8 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
                 bj = cd{10.0 / 12.0, -(hdt * (1.0 / (dx * dx)) + hdt * 10 / 12. * V[j])};
                 cj = (j + 1 < n) ? cd{1.0 / 12.0, -wj} : cd{0.0, 0.0};
             };
-            factorise<cd>(n, m, atab + CN_IB6 * L, atab + CN_H * L, atab + CN_G * L, 1.0, row);
+            factorise<cd>(n, m, atab + CN_IB6 * L, atab + CN_H * L, atab + CN_G * L, 1.0, maps, row);
         }
-        __syncthreads();
         chunk_products<cd>(m, atab + CN_H * L, atab + CN_G * L, atab + CN_F * L, atab + CN_GG * L);
         __syncthreads();
     }
@@ -502,6 +577,12 @@ extern "C" int mma_tdse_build_grids(const mma_tdse_grid* grids_dev, const mma_td
         if (mode == 0 && G.max_iter < 1) return MMA_ERR_ARG;
     }
     build_grids_kernel<<<n_grids, kThreads, 0, (cudaStream_t)stream>>>(grids_dev, mode);
+    return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+}
+
+int mma::ground_state_only(const mma_tdse_grid* grid_dev, cudaStream_t st)
+{
+    build_grids_kernel<<<1, kThreads, 0, st>>>(grid_dev, 2);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }
 

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/mma_tdse.h"
+#include "tdse_host.cuh"
 
 namespace {
 
@@ -133,7 +134,7 @@ extern "C" void Initialise_grid_and_ground_state(inputs_def* in)
         free_grid(g);
         return;
     }
-    rc = mma_tdse_build_grids(g.d, &g.h, 1, 0, nullptr);
+    rc = mma::ground_state_only(g.d, nullptr);  // call1DTDSE builds the step's tables for its own dt
     if (rc != MMA_OK) {
         set_status(rc, "grid build launch failed");
         free_grid(g);

@@ -15,7 +15,11 @@ enum { GS_IB12 = 0, GS_H, GS_F, GS_G, GS_GG, GS_SLOTS };
 constexpr int ADJ_SLOTS = 5;
 
 __device__ __forceinline__ double soft_coulomb(double x, double a) { return -1.0 / sqrt(a * a + x * x); }
-__device__ __forceinline__ double minus_grad_v(double x, double a) { return x * pow(a * a + x * x, -1.5); }
+__device__ __forceinline__ double minus_grad_v(double x, double a)
+{
+    const double s = a * a + x * x;  // x s^{-3/2} (tools.c:108-113)
+    return x / (s * sqrt(s));
+}
 
 __device__ __forceinline__ int64_t qidx(int64_t j, int64_t m) { return (j % m) * kThreads + (j / m); }
 
