@@ -42,11 +42,18 @@ typedef struct mma_hankel_problem {
  *           n_planes = number of slots in use (0..n_planes-1, each used once)
  *   planes  [n_planes][n_rho][n_omega] complex128 (or NULL)    per-plane transforms */
 
-/* Plain form: the reference's arithmetic in FP64, one J0 (CUDA j0) per (w, k, rho, r)
- * term.  One CTA per frequency. */
+/* Plain form: FP64 throughout.  FF contracts z first through the multiplication theorem (terms
+ * taken until the dropped tail is below 1e-17) where at most two planes are wanted and that is the
+ * smaller number of operations; else one J0 per (w, k, rho, r) term.  n_rho <= 2048.  The workspace
+ * is allocated and freed on the stream; mma_hankel_plain_ws takes it from the caller. */
 int mma_hankel_plain(const mma_hankel_problem *p, const double *ogrid, const double *rgrid, const double *zgrid,
                      const double *rho, const void *source, const double *pre, double *ff,
                      const int64_t *plane_slot, int n_planes, double *planes, void *stream);
+size_t mma_hankel_plain_scratch_bytes(const mma_hankel_problem *p);
+int mma_hankel_plain_ws(const mma_hankel_problem *p, const double *ogrid, const double *rgrid, const double *zgrid,
+                        const double *rho, const void *source, const double *pre, double *ff,
+                        const int64_t *plane_slot, int n_planes, double *planes, void *scratch,
+                        size_t scratch_bytes, void *stream);
 
 /* Parameters of the fast form, chosen on the host from the grids by mma_hankel_fast_plan. */
 typedef struct mma_hankel_fast_plan_t {

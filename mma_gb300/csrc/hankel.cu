@@ -1,4 +1,4 @@
-// hankel.cu -- far-field (Hankel) kernels: the plain FP64 form and the fast form.
+// hankel.cu -- far-field (Hankel) kernels of the fast form (the FP64 form: hankel_plain.cu).
 //
 // Reference: Hankel/Hankel_transform.py:452-519 (HankelTransform), :523-686 (Hankel_long).
 // Per plane k and frequency w (k_w = w/c, D_k = distance - z_k):
@@ -20,68 +20,7 @@ namespace mma {
 namespace hk {
 
 constexpr int kThreads = 256;
-constexpr int kMaxRhoPerThread = 8;  // plain form: n_rho <= 2048
 constexpr uint64_t kRingWaitNs = 2000000000ull;  // bounded waits of the ring stage 1 (2 s)
-
-// ------------------------------------------------------------------------ plain FP64 form
-// One CTA per frequency; per plane the CTA builds A_k[r] in shared memory, then each thread
-// accumulates its rho values with CUDA's FP64 j0, in the reference's argument order
-// k * r * rho / D.  The z-trapezoid is accumulated in registers (deterministic order).
-__global__ void __launch_bounds__(kThreads) plain_kernel(mma_hankel_problem P, const double* og, const double* rg,
-                                                         const double* zg, const double* rho, const void* src,
-                                                         const double2* pre, double2* ff, const int64_t* slot,
-                                                         double2* planes)
-{
-    extern __shared__ double2 A[];  // n_r
-    const int64_t o = blockIdx.x;
-    const int64_t Nr = P.n_r, Nz = P.n_z, Nrho = P.n_rho, No = P.n_omega;
-    const double k = og[o] / kC;
-    double2 acc[kMaxRhoPerThread];
-#pragma unroll
-    for (int q = 0; q < kMaxRhoPerThread; q++) acc[q] = make_double2(0.0, 0.0);
-    for (int64_t kz = 0; kz < Nz; kz++) {
-        const double D = P.distance - zg[kz];
-        const double tau = trap_w(zg, kz, Nz);
-        __syncthreads();
-        for (int64_t r = threadIdx.x; r < Nr; r += blockDim.x) {
-            const double rr = rg[r];
-            const double2 s = load_src_d(src, kz * P.plane_stride + o * P.omega_stride + r, P.source_c128);
-            double2 a = pre_at(P, pre, kz, o, r);  // the radial factor first, as in :505-512
-            if (P.near_field) {  // exp(-1j k r^2 / (2 D)), Hankel_transform.py:506
-                double sn, cs;
-                sincos(-((k * (rr * rr)) / (2.0 * D)), &sn, &cs);
-                a = make_double2(a.x * cs - a.y * sn, a.x * sn + a.y * cs);
-            }
-            a = make_double2(a.x * rr, a.y * rr);
-            a = make_double2(a.x * s.x - a.y * s.y, a.x * s.y + a.y * s.x);
-            const double w = trap_w(rg, r, Nr);
-            A[r] = make_double2(a.x * w, a.y * w);
-        }
-        __syncthreads();
-        const int64_t sl = slot ? slot[kz] : -1;
-#pragma unroll
-        for (int q = 0; q < kMaxRhoPerThread; q++) {
-            const int64_t j = threadIdx.x + (int64_t)q * blockDim.x;
-            if (j < Nrho) {
-                const double rj = rho[j];
-                double re = 0.0, im = 0.0;
-                for (int64_t r = 0; r < Nr; r++) {
-                    const double J = j0(k * rg[r] * rj / D);
-                    re = fma(A[r].x, J, re);
-                    im = fma(A[r].y, J, im);
-                }
-                if (sl >= 0 && planes) planes[(sl * Nrho + j) * No + o] = make_double2(re, im);
-                acc[q].x = fma(tau, re, acc[q].x);
-                acc[q].y = fma(tau, im, acc[q].y);
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < kMaxRhoPerThread; q++) {
-        const int64_t j = threadIdx.x + (int64_t)q * blockDim.x;
-        if (j < Nrho) ff[j * No + o] = acc[q];
-    }
-}
 
 // ------------------------------------------------------------------------ fast form, stage 1
 // Per-plane constants, independent of frequency, computed once per call (rows of MM + 4 floats):
@@ -827,22 +766,6 @@ static int g_stage1_mode = 1;
 // Test of the ring's bounded waits: when set, the ring's copies are never issued (every wait of
 // the call runs out after kRingWaitNs; the far field is NaN and the status word reports it).
 static int g_ring_no_issue = 0;
-
-extern "C" int mma_hankel_plain(const mma_hankel_problem* p, const double* ogrid, const double* rgrid,
-                                const double* zgrid, const double* rho, const void* source, const double* pre,
-                                double* ff, const int64_t* plane_slot, int n_planes, double* planes, void* stream)
-{
-    if (!valid(p) || !ogrid || !rgrid || !zgrid || !rho || !source || !ff) return MMA_ERR_ARG;
-    if (p->n_rho > (int64_t)kThreads * kMaxRhoPerThread) return MMA_ERR_TOO_LARGE;
-    if ((n_planes > 0) != (plane_slot != nullptr && planes != nullptr)) return MMA_ERR_ARG;
-    const size_t smem = sizeof(double2) * (size_t)p->n_r;
-    if (smem > 220 * 1024) return MMA_ERR_TOO_LARGE;
-    cudaFuncSetAttribute(plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    plain_kernel<<<(unsigned)p->n_omega, kThreads, smem, (cudaStream_t)stream>>>(
-        *p, ogrid, rgrid, zgrid, rho, source, reinterpret_cast<const double2*>(pre), reinterpret_cast<double2*>(ff),
-        n_planes > 0 ? plane_slot : nullptr, reinterpret_cast<double2*>(planes));
-    return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
-}
 
 extern "C" int mma_hankel_fast_plan(const double* zg, int64_t nz, double distance, double omega_max, double r_max,
                                     double rho_max, double tol, mma_hankel_fast_plan_t* plan)

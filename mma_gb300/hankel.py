@@ -14,8 +14,8 @@ Same names, arguments and results as the reference module:
   returning (pre_factor(kz) -> [Nr, No], exp_renorm(kz) -> [No]) like the reference.
 * ``HankelTransform`` (:452-519) -> [No, Nrho] complex128.
 * ``Hankel_long`` (:523-686) -- FF_integrated [Nrho, No], entry/exit planes,
-  cumulative results.  ``form="plain"`` runs the reference's arithmetic in FP64
-  (CUDA kernels in mma_gb300/csrc/hankel.cu); ``form="fast"`` runs the chosen
+  cumulative results.  ``form="plain"`` runs in FP64
+  (CUDA kernels in mma_gb300/csrc/hankel_plain.cu); ``form="fast"`` runs the chosen
   form (Bessel multiplication theorem, z-first contraction, FP32 with float-float
   phases) and records its truncation bound in ``self.fast_plan``.
 
@@ -64,6 +64,11 @@ def _sig():
     lib.mma_hankel_plain.argtypes = [P, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                      c_void_p, c_int, c_void_p, c_void_p]
     lib.mma_hankel_plain.restype = c_int
+    lib.mma_hankel_plain_scratch_bytes.argtypes = [P]
+    lib.mma_hankel_plain_scratch_bytes.restype = c_size_t
+    lib.mma_hankel_plain_ws.argtypes = [P, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                        c_void_p, c_int, c_void_p, c_void_p, c_size_t, c_void_p]
+    lib.mma_hankel_plain_ws.restype = c_int
     lib.mma_hankel_fast_plan.argtypes = [POINTER(c_double), c_int64, c_double, c_double, c_double, c_double,
                                          c_double, POINTER(FastPlan)]
     lib.mma_hankel_fast_plan.restype = c_int
@@ -524,9 +529,11 @@ def _far_field_on(lib, strm, prob, S, ogrid, rgrid, zgrid, rho, distance, pre_ta
     ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
     plan_d = None
     if form == "plain":
-        _check(lib.mma_hankel_plain(ctypes.byref(prob), og.data_ptr(), rg.data_ptr(), zg.data_ptr(), rh.data_ptr(),
-                                    S.data_ptr(), ptr(pre), ff.data_ptr(), ptr(slot), len(planes), ptr(pl), st),
-               "mma_hankel_plain")
+        nb = int(lib.mma_hankel_plain_scratch_bytes(ctypes.byref(prob)))
+        scratch = torch.empty(nb, dtype=torch.uint8, device=dev)
+        _check(lib.mma_hankel_plain_ws(ctypes.byref(prob), og.data_ptr(), rg.data_ptr(), zg.data_ptr(), rh.data_ptr(),
+                                       S.data_ptr(), ptr(pre), ff.data_ptr(), ptr(slot), len(planes), ptr(pl),
+                                       scratch.data_ptr(), nb, st), "mma_hankel_plain")
     elif form == "fast":
         zh = np.ascontiguousarray(_np(zgrid), dtype=np.float64)
         plan = FastPlan()
