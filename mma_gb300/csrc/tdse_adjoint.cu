@@ -12,11 +12,13 @@
 // A^H solved with its own factorisation (build_grids_kernel, adj_tab) by the same
 // partitioned solve.  The forward pass stores psi every K steps (ckpt_*); going backwards,
 // each segment is recomputed forwards from its checkpoint into a per-CTA history, then
-// swept backwards.  Cost: about three forward passes.
+// swept backwards.  Cost: about three forward passes.  Batches that leave SMs idle spread each
+// instance over a thread-block cluster (adjoint_cluster_kernel).
 #include <cuda_runtime.h>
 
 #include "../../include/mma_tdse.h"
 #include "common.cuh"
+#include "tdse_cluster.cuh"
 #include "tdse_solver.cuh"
 #include "tdse_step.cuh"
 
@@ -207,10 +209,397 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_fp64_kernel(Args P)
     }
 }
 
+// ---------------------------------------------------------------------------- adjoint sweep, cluster
+// The same sweep with an instance spread over a cluster (tdse_cluster.cu has the scheme).  lambda, psi
+// and the sweep buffer stay in shared memory with the tables of the phase at hand: the step's while a
+// segment is recomputed, those of A^H while it is swept back (reloaded from L2 once per segment).
+// An adjoint step needs two cluster barriers: z beside the chunk is known without an exchange, on the
+// right as the carry z_in of the backward scan, on the left as y_in - g z_first (y_in the carry of the
+// forward scan), so lambda_k = 2 M2 z - mu - 2 a_k gv psi_k follows in the pass that makes z.
+// Bound by the FP64 pipe: about 30 + 40 operations per site and step and 200 per thread.
+// Per step of one 8001-site instance: 269 us on one CTA, 23 us on a cluster of 16; 64 instances 272 ->
+// 114 us (36 clusters of 4).
+struct ClusterArgs {
+    Args A;
+    int m_cap;
+    int64_t hist_stride;  // complex entries of one state in a cluster's history
+};
+
+constexpr int kGradRing = 8;
+
+__host__ __device__ inline size_t adj_site_bytes() { return 6 * 16; }
+__host__ __device__ inline size_t adj_fixed_bytes(int nc)
+{
+    using namespace clk;
+    const size_t nw = (size_t)nc * kW;
+    return 16 * (2 * nw + 2 * kW * nw + 2 * kPhSteps * kPh) + 8 * kGradRing * nw;
+}
+
+__global__ void __launch_bounds__(clk::kT, 1) adjoint_cluster_kernel(ClusterArgs Q)
+{
+    using namespace clk;
+    typedef Fp64 N;
+    const Args& P = Q.A;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int NC = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), NW = NC * kW;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, g = rank * kW + w;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int ML = Q.m_cap * kT;
+    cd* const lam = reinterpret_cast<cd*>(smem);
+    cd *const psi = lam + ML, *const yv = psi + ML, *const ib = yv + ML, *const hh = ib + ML, *const gg = hh + ML;
+    cd *const totF = gg + ML, *const totB = totF + NW, *const wtF = totB + NW, *const wtB = wtF + kW * NW,
+              *const phs = wtB + kW * NW;
+    double* const ring = reinterpret_cast<double*>(phs + 2 * kPhSteps * kPh);
+    Scan<N> scan(cluster, totF, totB, wtF, wtB);
+    __shared__ cd edge[2];
+    __shared__ int s_inst;
+    __shared__ long long s_gate;
+
+    for (;;) {
+        cluster.sync();
+        if (rank == 0 && t == 0) {
+            const int v = atomicAdd(P.counter, 1);
+            for (int r = 0; r < NC; r++) *cluster.map_shared_rank(&s_inst, r) = v;
+        }
+        cluster.sync();
+        const int inst = s_inst;
+        if (inst >= P.n_inst) break;
+        const mma_tdse_instance I = P.insts[inst];
+        const mma_tdse_grid G = P.grids[I.grid];
+        const int64_t S = I.n_steps, K = I.ckpt_every;
+        const int n = (int)G.n, m256 = (int)G.m;
+        const int64_t L = G.m * kThreads;
+        const cd* ctab = reinterpret_cast<const cd*>(G.cn_tab);
+        const cd* atab = reinterpret_cast<const cd*>(G.adj_tab);
+        const double* f = P.fields + I.field_off;
+        const double* ai = P.a + P.a_off[inst];
+        double* gi = P.grad + P.grad_off[inst];
+        const double dt = G.dt, dx = G.dx, x0 = G.x[0];
+        const int m = (n + NC * kT - 1) / (NC * kT);
+        if (L > P.max_L || m > Q.m_cap || K > P.max_K) {  // wider than the launch was sized for
+            for (int64_t e = (int64_t)rank * kT + t; e < S; e += NC * kT) gi[e] = __longlong_as_double(0x7ff8000000000000LL);
+            continue;
+        }
+        const int c0 = rank * kT + t, s0 = c0 * m;
+        // this cluster's history, [state][site of the chunk][chunk]
+        cd* const hist = P.scratch + (int64_t)(blockIdx.x / NC) * (P.max_K + 1) * Q.hist_stride + c0;
+        const int64_t row = NC * kT;
+        auto hst = [&](int64_t h, int i) { return hist + h * Q.hist_stride + i * row; };
+        if (t == 0) {
+            s_gate = S;
+            // the grid's ends; every other edge comes from its neighbour, perhaps already
+            if (rank == 0) edge[0] = N::zero();
+            if (rank == NC - 1) edge[1] = N::zero();
+        }
+        __syncthreads();
+        for (int64_t b = 0; b < S; b += kT) {
+            const int64_t k = b + t;
+            bool hit = false;
+            if (k < S) {
+                double fa = (k < I.n_field) ? f[k] : 0.0, fb = (k + 1 < I.n_field) ? f[k + 1] : 0.0;
+                if (fabs(fa) <= I.gate_floor) fa = 0.0;
+                if (fabs(fb) <= I.gate_floor) fb = 0.0;
+                hit = fa * fb <= 0.0;
+                if (hit) atomicMin(&s_gate, (long long)k);
+            }
+            if (__syncthreads_or(hit)) break;
+        }
+        __syncthreads();
+        const int64_t gate = s_gate;
+        auto applied = [&](int64_t k) { return (k < 0 || k <= gate || k >= I.n_field) ? 0.0 : f[k]; };
+        // the tables of the step (tab = cn_tab) or of A^H, and the scans' constants for them; returns g
+        // of the site before the chunk.  Contains cluster barriers.
+        auto load_tables = [&](const cd* tab) {
+            cd cF = N::one(), cB = N::one(), gprev = N::zero();
+            for (int i = 0; i < m; i++) {
+                const int j = s0 + i, q = i * kT + t;
+                cd a = N::zero(), h = a, gq = a;
+                if (j < n) {
+                    const int64_t e = (int64_t)(j % m256) * kThreads + j / m256;
+                    a = tab[CN_IB6 * L + e];
+                    h = tab[CN_H * L + e];
+                    gq = tab[CN_G * L + e];
+                }
+                ib[q] = a;
+                hh[q] = h;
+                gg[q] = gq;
+                cF = N::mul(cF, N::neg(h));
+                cB = N::mul(cB, N::neg(gq));
+            }
+            if (s0 > 0 && s0 - 1 < n)
+                gprev = tab[CN_G * L + (int64_t)((s0 - 1) % m256) * kThreads + (s0 - 1) / m256];
+            scan.setup(cluster, cF, cB);
+            return gprev;
+        };
+        auto send_edges = [&] {
+            if (t == 0 && rank > 0) *cluster.map_shared_rank(&edge[1], rank - 1) = psi[0];
+            if (t == kT - 1 && rank + 1 < NC) *cluster.map_shared_rank(&edge[0], rank + 1) = psi[(m - 1) * kT + t];
+        };
+        // phases of the steps k0, k0 + dir, ... into half `b` of the table: e^{i F dt x} at site `site` of
+        // the warps' first chunks and the factors between chunks, then e^{-dir' i F dt dx}
+        auto phases = [&](int64_t k0, int dir, int site, int half) {
+            if (t >= kPhSteps * kPh) return;
+            const int a = t % kPh;
+            const int64_t k = k0 + dir * (t / kPh);
+            const double Fdt = (k < S ? applied(k) : 0.0) * dt, step = (double)m * dx;
+            double ang;
+            if (a < kPhA) ang = Fdt * (step * (4 * a));
+            else if (a < kPhA + kPhB) ang = Fdt * (step * (a - kPhA));
+            else if (a < kPh - 1) ang = Fdt * (x0 + dx * (double)((rank * kT + 32 * (a - kPhA - kPhB)) * m + site));
+            else ang = -(double)dir * (Fdt * dx);
+            double sn, cs;
+            sincos(ang, &sn, &cs);
+            phs[half * kPhSteps * kPh + t] = cd{cs, sn};
+        };
+        auto start_phase = [&](const cd* ps) {
+            return cmul(cmul(ps[lane >> 2], ps[kPhA + (lane & 3)]), ps[kPhA + kPhB + w]);
+        };
+        for (int i = 0; i < m; i++) lam[i * kT + t] = N::zero();  // lambda_S = 0
+        // rank 0: the gradient of steps k, k - 1, ... (cnt of them) from ring slots slot0, slot0 + 1, ...
+        auto flush = [&](int64_t k, int cnt) {
+            if (t < 4 * cnt) {
+                const int sl = t / 4;
+                double s = 0.0;
+                for (int q = t % 4; q < NW; q += 4) s += ring[sl * NW + q];
+                s += __shfl_xor_sync(__activemask(), s, 1);
+                s += __shfl_xor_sync(__activemask(), s, 2);
+                if (t % 4 == 0) gi[k - sl] = ai[k - sl + 1] - dt * s;
+            }
+        };
+
+        const int64_t nseg = (S + K - 1) / K;
+        for (int64_t c = nseg - 1; c >= 0; c--) {
+            const int64_t k0 = c * K, k1 = (k0 + K < S) ? k0 + K : S;
+            // ---- recompute states k0 .. k1 into the history
+            const double* cp = P.ckpts + I.ckpt_off + c * 2 * n;
+            for (int i = 0; i < m; i++) {
+                const int j = s0 + i;
+                const cd v = (j < n) ? ld2(cp + 2 * j) : N::zero();
+                psi[i * kT + t] = v;
+                *hst(0, i) = v;
+            }
+            send_edges();
+            phases(k0, 1, m - 1, 0);
+            load_tables(ctab);  // its barriers also publish the edges and the phases
+            for (int64_t k = k0; k < k1; k++) {
+                const int64_t e = k - k0;
+                const int kp = (int)(e % kPhSteps);
+                cd pm = (t == 0) ? edge[0] : psi[(m - 1) * kT + t - 1];
+                const cd nx = (t == kT - 1) ? edge[1] : psi[t + 1];
+                cd pc = psi[t];
+                cd b = N::zero();
+#pragma unroll 2
+                for (int i = 0; i < m; i++) {
+                    const int q = i * kT + t;
+                    const cd pn = (i + 1 < m) ? psi[q + kT] : nx;
+                    const cd r = N::rhs(ib[q], pc, pm, pn);
+                    yv[q] = r;
+                    b = cfms(hh[q], b, r);
+                    pm = pc;
+                    pc = pn;
+                }
+                b = scan.forward_out(cluster, b);
+                cluster.barrier_arrive();
+                if (kp == kPhSteps - 1) phases(k + 1, 1, m - 1, (int)((e / kPhSteps + 1) % 2));
+                cd bx = N::shup(b, 1);
+                cluster.barrier_wait();
+                cd y = scan.forward_in(bx);
+#pragma unroll 2
+                for (int i = 0; i < m; i++) {
+                    const int q = i * kT + t;
+                    y = cfms(hh[q], y, yv[q]);
+                    yv[q] = y;
+                }
+                b = y;
+#pragma unroll 2
+                for (int i = m - 2; i >= 0; i--) {
+                    const int q = i * kT + t;
+                    b = cfms(gg[q], b, yv[q]);
+                }
+                b = scan.backward_out(cluster, b);
+                cluster.barrier_arrive();
+                bx = N::shdn(b, 1);
+                const cd* ps = phs + ((int)(e / kPhSteps % 2) * kPhSteps + kp) * kPh;
+                cd ph = start_phase(ps);
+                const cd zc = ps[kPh - 1];
+                cluster.barrier_wait();
+                cd u = scan.backward_in(bx);
+#pragma unroll 2
+                for (int i = m - 1; i >= 0; i--) {
+                    const int q = i * kT + t;
+                    u = cfms(gg[q], u, yv[q]);
+                    const cd pn = N::update(ph, u, psi[q]);
+                    psi[q] = pn;
+                    *hst(e + 1, i) = pn;
+                    ph = cmul(ph, zc);
+                }
+                send_edges();
+                cluster.sync();
+            }
+            // ---- adjoint steps k = k1 - 1 .. k0; psi holds state k + 1
+            phases(k1 - 1, -1, 0, 0);
+            const cd gprev = load_tables(atab);
+            for (int64_t k = k1 - 1; k >= k0; k--) {
+                const int64_t e = k1 - 1 - k;
+                const int kp = (int)(e % kPhSteps);
+                const double ak2 = -2.0 * ai[k];
+                const cd* ps = phs + ((int)(e / kPhSteps % 2) * kPhSteps + kp) * kPh;
+                cd ph = start_phase(ps);
+                const cd z = ps[kPh - 1];
+                // gradient term, mu = conj(Phi) lambda, forward sweep of A^H z = mu
+                double gsum = 0.0;
+                cd b = N::zero();
+#pragma unroll 2
+                for (int i = 0; i < m; i++) {
+                    const int q = i * kT + t;
+                    const cd l = lam[q], p = psi[q];
+                    const double x = x0 + dx * (double)(s0 + i);
+                    gsum = fma(x, fma(l.re, p.im, -l.im * p.re), gsum);  // x Im(conj(l) p)
+                    const cd mu{fma(ph.re, l.re, ph.im * l.im), fma(ph.re, l.im, -ph.im * l.re)};
+                    ph = cmul(ph, z);
+                    lam[q] = mu;
+                    const cd r = cmul(ib[q], mu);
+                    yv[q] = r;
+                    b = cfms(hh[q], b, r);
+                }
+                b = scan.forward_out(cluster, b);
+#pragma unroll
+                for (int d = 16; d >= 1; d >>= 1) gsum += shfl_xor(gsum, d);
+                if (lane == 0) cluster.map_shared_rank(ring, 0)[(int)(e % kGradRing) * NW + g] = gsum;
+                cluster.barrier_arrive();
+                if (kp == kPhSteps - 1) phases(k - 1, -1, 0, (int)((e / kPhSteps + 1) % 2));
+                cd bx = N::shup(b, 1);
+                cluster.barrier_wait();
+                if (rank == 0 && (e % kGradRing == kGradRing - 1 || k == k0))
+                    flush(k + e % kGradRing, (int)(e % kGradRing) + 1);
+                const cd yin = scan.forward_in(bx);
+                cd y = yin;
+#pragma unroll 2
+                for (int i = 0; i < m; i++) {
+                    const int q = i * kT + t;
+                    y = cfms(hh[q], y, yv[q]);
+                    yv[q] = y;
+                }
+                b = y;
+#pragma unroll 2
+                for (int i = m - 2; i >= 0; i--) {
+                    const int q = i * kT + t;
+                    b = cfms(gg[q], b, yv[q]);
+                }
+                b = scan.backward_out(cluster, b);
+                cluster.barrier_arrive();
+                bx = N::shdn(b, 1);
+                // psi_k and -V' of the next site, one iteration ahead of their use
+                cd pre_p;
+                double pre_v;
+                auto prefetch = [&](int i) {
+                    const int j = s0 + i < n ? s0 + i : n - 1;
+                    pre_p = *hst(k - k0, i);
+                    pre_v = ctab[CN_GVX * L + (int64_t)(j % m256) * kThreads + j / m256].re;
+                };
+                prefetch(m - 1);
+                cluster.barrier_wait();
+                // z from the exact carry; lambda_k = 2 M2 z - mu - 2 a_k gv psi_k one site behind it
+                cd zn = scan.backward_in(bx), zc = cfms(gg[(m - 1) * kT + t], zn, yv[(m - 1) * kT + t]);
+#pragma unroll 2
+                for (int i = m - 1; i >= 0; i--) {
+                    const int q = i * kT + t, j = s0 + i;
+                    const cd zm = i > 0 ? cfms(gg[q - kT], zc, yv[q - kT]) : cfms(gprev, zc, yin);
+                    const cd p = pre_p, mu = lam[q];
+                    const double v = ak2 * pre_v;
+                    if (i > 0) prefetch(i - 1);
+                    cd l = N::zero();
+                    if (j < n) {
+                        l = cd{fma(v, p.re, fma(1.0 / 6.0, fma(10.0, zc.re, zm.re + zn.re), -mu.re)),
+                               fma(v, p.im, fma(1.0 / 6.0, fma(10.0, zc.im, zm.im + zn.im), -mu.im))};
+                    }
+                    lam[q] = l;
+                    psi[q] = p;  // state k, the next step's psi_{k+1}
+                    zn = zc;
+                    zc = zm;
+                }
+            }
+            cluster.sync();  // the last step's carries are read before the next tables' constants replace them
+        }
+    }
+}
+
 }  // namespace adj
 }  // namespace mma
 
 using namespace mma;
+
+namespace {
+
+// Expected us per step (recompute and adjoint) of the whole batch, fitted to runs (measured / model):
+// one CTA 301 sites 41.9 / 41.7, 2001 sites 85.5 / 87.3, 8001 sites 269 / 270; cluster 8001 sites
+// NC = 4 55.6 / 54.2, 8 33.4 / 32.6, 16 23.0 / 21.8, 301 sites NC = 4 13.1 / 13.7.
+double adj_one_cta_us(int m256, int n_inst, int sms) { return (double)((n_inst + sms - 1) / sms) * (26.5 + 7.6 * m256); }
+double adj_cluster_us(int m, int n_inst, int run, int nc, int sms)
+{
+    const int full = n_inst / run, rest = n_inst % run;
+    const double one = 11.0 + 2.7 * m, two = 1.25 * one;  // two CTAs of the launch on an SM: 1.1 to 1.5 measured
+    return full * (run * nc > sms ? two : one) + (rest == 0 ? 0.0 : rest * nc > sms ? two : one);
+}
+
+cudaLaunchConfig_t adj_config(int nc, int clusters, size_t smem, cudaStream_t st, cudaLaunchAttribute* at)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(clusters * nc));
+    cfg.blockDim = dim3(clk::kT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = (unsigned)nc;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+struct AdjCluster {
+    int nc, m, clusters;
+    size_t smem;
+};
+
+// The cluster size with the least expected time, or false where one CTA per instance is expected to
+// finish sooner.  A cluster's history needs (K + 1) states in the caller's scratch.
+bool choose_adj_cluster(int max_m, int K, int n_inst, int sms, size_t scratch_bytes, AdjCluster* out)
+{
+    auto kern = adj::adjoint_cluster_kernel;
+    double best = adj_one_cta_us(max_m, n_inst, sms);
+    bool found = false;
+    for (int nc = clk::kMaxNC; nc >= 1; nc--) {
+        const int m = (max_m * kThreads + nc * clk::kT - 1) / (nc * clk::kT);
+        const size_t smem = (size_t)m * clk::kT * adj::adj_site_bytes() + adj::adj_fixed_bytes(nc);
+        const size_t hist = sizeof(cd) * (size_t)(K + 1) * nc * clk::kT * m;
+        if (smem > 226 * 1024 || (nc > 1 && (nc - 1) * m * clk::kT >= max_m * kThreads) || scratch_bytes < hist) continue;
+        int run = sms * (smem > 112 * 1024 ? 1 : 2) / nc;  // if every SM could be filled
+        if ((size_t)run > scratch_bytes / hist) run = (int)(scratch_bytes / hist);
+        if (run > n_inst) run = n_inst;
+        if (run < 1 || adj_cluster_us(m, n_inst, run, nc, sms) >= best) continue;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            return false;
+        cudaLaunchAttribute at{};
+        cudaLaunchConfig_t cfg = adj_config(nc, 1, smem, nullptr, &at);
+        int active = 0;
+        if (cudaOccupancyMaxActiveClusters(&active, kern, &cfg) != cudaSuccess || active < 1) {
+            cudaGetLastError();
+            continue;
+        }
+        if (run > active) run = active;
+        const double us = adj_cluster_us(m, n_inst, run, nc, sms);
+        if (us < best) {
+            best = us;
+            *out = AdjCluster{nc, m, run, smem};
+            found = true;
+        }
+    }
+    return found;
+}
+
+}  // namespace
 
 extern "C" int mma_tdse_loss_grad(const mma_tdse_instance* insts, int n_inst, const double* outputs,
                                   const double* tmax, double dt, double w_lo, double w_hi, double* loss, double* a,
@@ -258,6 +647,18 @@ extern "C" int mma_tdse_adjoint(const mma_tdse_instance* insts, int n_inst, cons
     if (cudaMemsetAsync(bufs->counter, 0, sizeof(int), st) != cudaSuccess) return MMA_ERR_CUDA;
     adj::Args A{insts, n_inst, grids, bufs->fields, bufs->snapshots, a, a_off, grad, grad_off, bufs->counter,
                 reinterpret_cast<cd*>(bufs->scratch), (int64_t)max_m * kThreads, (int64_t)max_ckpt_every};
+    // a caller that asks for fewer CTAs than the batch could use keeps the one-CTA kernel and that limit
+    const bool limited = grid_ctas < n_inst && grid_ctas < sms;
+    AdjCluster ac;
+    if (!limited && choose_adj_cluster(max_m, max_ckpt_every, n_inst, sms, bufs->scratch_bytes, &ac)) {
+        adj::ClusterArgs Q{A, ac.m, (int64_t)ac.nc * clk::kT * ac.m};
+        auto kern = adj::adjoint_cluster_kernel;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ac.smem) != cudaSuccess)
+            return MMA_ERR_CUDA;
+        cudaLaunchAttribute at{};
+        cudaLaunchConfig_t cfg = adj_config(ac.nc, ac.clusters, ac.smem, st, &at);
+        return cudaLaunchKernelEx(&cfg, kern, Q) == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+    }
     cudaFuncSetAttribute(adj::adjoint_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     adj::adjoint_fp64_kernel<<<grid_ctas, kThreads, smem, st>>>(A);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;

@@ -23,25 +23,14 @@
 // and step, one warp per sub-partition) or by the latency of the scans (float-float); per step, one
 // CTA -> cluster: one 8001-site instance 108.8 -> 11.6 us in FP64 and 35.1 -> 5.4 us in float-float
 // (NC = 16), 601 sites 24.3 -> 6.7 us (FP64, NC = 8), 24 float-float instances 35.3 -> 8.8 us.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
-#include "../../include/mma_tdse.h"
-#include "common.cuh"
-#include "df64.cuh"
+#include "tdse_cluster.cuh"
 #include "tdse_host.cuh"
-#include "tdse_step.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace mma {
 namespace clk {
 
-constexpr int kT = 128, kW = kT / 32;  // one warp per sub-partition: FP64 issue is the limit, not latency
-constexpr int kMaxNC = 16;  // the largest cluster the hardware takes (over 8: opt-in)
-constexpr int kPhA = 8, kPhB = 4;  // lane = 4 a + b: e^{i F dt (4 a m dx)}, e^{i F dt (b m dx)}
-constexpr int kPh = kPhA + kPhB + kW + 1;  // + the warps' start phases + e^{-i F dt dx}
-constexpr int kPhSteps = kT / kPh;         // steps whose phases one pass of the CTA computes
 constexpr int kRing = 8, kObs = 5;         // steps of observables collected before they are summed
 constexpr int kGroups = 3;                 // thread groups that share those sums (kGroups kRing kObs <= kT)
 
@@ -56,121 +45,6 @@ struct Args {
     int* counter;
     int m_cap;      // sites per thread the shared memory was sized for
     int64_t max_L;  // widest grid of the launch (padded sites), as the caller stated it
-};
-
-// ------------------------------------------------------------------ arithmetic of the two forms
-struct Fp64 {
-    typedef cd C;
-    typedef double R;  // a partial sum
-    static constexpr bool kFp64 = true;
-    static __device__ const C* table(const mma_tdse_grid& G) { return reinterpret_cast<const C*>(G.cn_tab); }
-    static __device__ C zero() { return cd{0.0, 0.0}; }
-    static __device__ C one() { return cd{1.0, 0.0}; }
-    static __device__ C neg(C a) { return cd{-a.re, -a.im}; }
-    static __device__ C conj(C a) { return cd{a.re, -a.im}; }
-    static __device__ bool tiny(C a) { return fabs(a.re) + fabs(a.im) < 1e-40; }
-    static __device__ C mul(C a, C b) { return cmul(a, b); }
-    static __device__ C fma(C a, C b, C z) { return cfma(a, b, z); }
-    static __device__ C fms(C a, C b, C z) { return cfms(a, b, z); }
-    static __device__ C rhs(C ib, C p, C a, C b)
-    {
-        return cmul(ib, cd{::fma(10.0, p.re, a.re + b.re), ::fma(10.0, p.im, a.im + b.im)});
-    }
-    static __device__ C update(C ph, C u, C p) { return cmul(ph, u - p); }
-    static __device__ C shup(C v, int d) { return cd{shfl_up(v.re, d), shfl_up(v.im, d)}; }
-    static __device__ C shdn(C v, int d) { return cd{shfl_down(v.re, d), shfl_down(v.im, d)}; }
-    static __device__ C bcast(C v, int l) { return cd{shfl_idx(v.re, l), shfl_idx(v.im, l)}; }
-    static __device__ C from(double re, double im) { return cd{re, im}; }
-    static __device__ void to_d(C v, double& re, double& im) { re = v.re, im = v.im; }
-    static __device__ R re(C v) { return v.re; }
-    static __device__ bool has_im(C v) { return v.im != 0.0; }
-    static __device__ R rzero() { return 0.0; }
-    static __device__ R radd(R a, R b) { return a + b; }
-    static __device__ R rxor(R a, int d) { return shfl_xor(a, d); }
-    static __device__ double rd(R a) { return a; }
-    struct Acc {
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0, w = 0.0;
-        __device__ void add(C pn, C gx, R p0, bool in)
-        {
-            const double n2 = ::fma(pn.re, pn.re, pn.im * pn.im);
-            a0 = ::fma(n2, gx.re, a0);
-            a1 = ::fma(n2, gx.im, a1);
-            a2 = ::fma(pn.re, p0, a2);
-            a3 = ::fma(pn.im, p0, a3);
-            if (in) w += n2;
-        }
-        // the imaginary part of a complex ground state: <psi0|psi> += conj(i p0i) psi
-        __device__ void add_im(C pn, R p0i)
-        {
-            a2 = ::fma(pn.im, p0i, a2);
-            a3 = ::fma(-pn.re, p0i, a3);
-        }
-        __device__ void get(R (&v)[4]) { v[0] = a0, v[1] = a1, v[2] = a2, v[3] = a3; }
-        __device__ R window() { return w; }
-    };
-};
-
-struct Df64 {
-    typedef dfk::pk C;
-    typedef dfk::df R;
-    static constexpr bool kFp64 = false;
-    static __device__ const C* table(const mma_tdse_grid& G) { return reinterpret_cast<const C*>(G.df_tab); }
-    static __device__ C zero() { return C{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
-    static __device__ C one() { return C{make_float2(1.f, 0.f), make_float2(0.f, 0.f)}; }
-    static __device__ C neg(C a) { return C{dfk::ng2(a.h), dfk::ng2(a.l)}; }
-    static __device__ C conj(C a) { return C{make_float2(a.h.x, -a.h.y), make_float2(a.l.x, -a.l.y)}; }
-    static __device__ bool tiny(C a) { return fabsf(a.h.x) + fabsf(a.h.y) < 1e-36f; }
-    static __device__ C mul(C a, C b) { return dfk::cmul_p(a, b); }
-    static __device__ C fma(C a, C b, C z) { return dfk::cfma_p(a, b, z); }
-    static __device__ C fms(C a, C b, C z) { return dfk::cfms_p(a, b, z); }
-    static __device__ C rhs(C ib, C p, C a, C b) { return dfk::cmul_pu(ib, dfk::ten_sum_p(p, a, b)); }
-    static __device__ C update(C ph, C u, C p)
-    {
-        float2 s, t;
-        dfk::two_sum2(u.h, dfk::ng2(p.h), s, t);
-        return dfk::cmul_p(ph, C{s, dfk::add2(t, dfk::sub2(u.l, p.l))});
-    }
-    static __device__ C shup(C v, int d) { return dfk::pshup(v, d); }
-    static __device__ C shdn(C v, int d) { return dfk::pshdn(v, d); }
-    static __device__ C bcast(C v, int l)
-    {
-        return C{make_float2(__shfl_sync(0xffffffffu, v.h.x, l), __shfl_sync(0xffffffffu, v.h.y, l)),
-                 make_float2(__shfl_sync(0xffffffffu, v.l.x, l), __shfl_sync(0xffffffffu, v.l.y, l))};
-    }
-    static __device__ C from(double re, double im)
-    {
-        const dfk::df a = dfk::from_d(re), b = dfk::from_d(im);
-        return C{make_float2(a.hi, b.hi), make_float2(a.lo, b.lo)};
-    }
-    static __device__ void to_d(C v, double& re, double& im)
-    {
-        re = (double)v.h.x + (double)v.l.x;
-        im = (double)v.h.y + (double)v.l.y;
-    }
-    static __device__ R re(C v) { return R{v.h.x, v.l.x}; }
-    static __device__ bool has_im(C v) { return v.h.y != 0.f; }
-    static __device__ R rzero() { return R{0.f, 0.f}; }
-    static __device__ R radd(R a, R b) { return dfk::add(a, b); }
-    static __device__ R rxor(R a, int d) { return dfk::shfl_xor_df(a, d); }
-    static __device__ double rd(R a) { return dfk::to_d(a); }
-    struct Acc {
-        C a01 = zero(), a23 = zero();
-        R w = rzero();
-        __device__ void add(C pn, C gx, R p0, bool in)
-        {
-            const R n2 = dfk::norm2_u(pn);
-            dfk::acc_mul_p(a01, n2.hi, n2.lo, gx);
-            dfk::acc_mul_p(a23, p0.hi, p0.lo, pn);
-            if (in) w = dfk::add(w, dfk::renorm(n2.hi, n2.lo));
-        }
-        __device__ void add_im(C pn, R p0i) { dfk::acc_mul_p(a23, p0i.hi, p0i.lo, C{dfk::mipair(pn.h), dfk::mipair(pn.l)}); }
-        __device__ void get(R (&v)[4])
-        {
-            const C x = dfk::renorm2(a01.h, a01.l), y = dfk::renorm2(a23.h, a23.l);
-            v[0] = R{x.h.x, x.l.x}, v[1] = R{x.h.y, x.l.y}, v[2] = R{y.h.x, y.l.x}, v[3] = R{y.h.y, y.l.y};
-        }
-        __device__ R window() { return w; }
-    };
 };
 
 // Dynamic shared memory: per padded site psi, sweep, 1/(6 beta), h, g, (-V', x) [16 bytes each] and
@@ -200,6 +74,7 @@ __global__ void __launch_bounds__(kT, 1) propagate_cluster_kernel(Args P)
     R* const p0 = reinterpret_cast<R*>(phs + 2 * kPhSteps * kPh);
     R* const ring = p0 + ML;
     R* const part = ring + kRing * NW * kObs;
+    Scan<N> scan(cluster, totF, totB, wtF, wtB);
     __shared__ C edge[2];
     __shared__ int s_inst;
     __shared__ long long s_gate;
@@ -293,38 +168,7 @@ __global__ void __launch_bounds__(kT, 1) propagate_cluster_kernel(Args P)
         const bool warp_win = __any_sync(0xffffffffu, s0 <= hi && s0 + m > lo);
         auto applied = [&](int64_t k) { return (k <= gate || k >= I.n_field || k >= S) ? 0.0 : f[k]; };
 
-        // ---- constants of the scans: products of the chunk coefficients over 1, 2, 4, 8, 16 chunks
-        C f_lv[5], b_lv[5];
-#pragma unroll
-        for (int l = 0; l < 5; l++) {
-            f_lv[l] = cF;
-            b_lv[l] = cB;
-            const C up = N::shup(cF, 1 << l), dn = N::shdn(cB, 1 << l);
-            if (lane >= (1 << l)) cF = N::mul(cF, up);
-            if (lane + (1 << l) < 32) cB = N::mul(cB, dn);
-        }
-        const C wF = N::bcast(cF, 31), wB = N::bcast(cB, 0);
-        const C f_ex = N::shup(cF, 1), b_ex = N::shdn(cB, 1);  // products of the chunks before (after) this one
-        if (lane < NC) {
-            cluster.map_shared_rank(totF, lane)[g] = wF;
-            cluster.map_shared_rank(totB, lane)[g] = wB;
-        }
-        cluster.sync();
-        int KF = 0, KB = 0;
-        if (lane == 0) {
-            C W = N::one();
-            for (; KF < g && !N::tiny(W); KF++) {
-                wtF[w * NW + KF] = W;
-                W = N::mul(W, totF[g - 1 - KF]);
-            }
-            W = N::one();
-            for (; KB < NW - 1 - g && !N::tiny(W); KB++) {
-                wtB[w * NW + KB] = W;
-                W = N::mul(W, totB[g + 1 + KB]);
-            }
-        }
-        KF = __shfl_sync(0xffffffffu, KF, 0);
-        KB = __shfl_sync(0xffffffffu, KB, 0);
+        scan.setup(cluster, cF, cB);
         auto send_edges = [&] {
             if (t == 0 && rank > 0) *cluster.map_shared_rank(&edge[1], rank - 1) = psi[0];
             if (t == kT - 1 && rank + 1 < NC) *cluster.map_shared_rank(&edge[0], rank + 1) = psi[(m - 1) * kT + t];
@@ -433,23 +277,15 @@ __global__ void __launch_bounds__(kT, 1) propagate_cluster_kernel(Args P)
                 pm = pc;
                 pc = pn;
             }
-#pragma unroll
-            for (int l = 0; l < 5; l++) {
-                const C up = N::shup(b, 1 << l);
-                if (lane >= (1 << l)) b = N::fma(f_lv[l], up, b);
-            }
-            C tot = N::bcast(b, 31);
-            if (lane >= rank && lane < NC) cluster.map_shared_rank(totF, lane)[g] = tot;
+            b = scan.forward_out(cluster, b);
             cluster.barrier_arrive();
             const int kp = (int)(k % kPhSteps);
             if (kp == kPhSteps - 1) phases(k + 1);
             C bx = N::shup(b, 1);
             cluster.barrier_wait();
             if (rank == 0 && k > 0 && k % kRing == 0) flush(k - kRing, kRing);
-            C yw = N::zero();
-            for (int q = 0; q < KF; q++) yw = N::fma(wtF[w * NW + q], totF[g - 1 - q], yw);
             // ---- forward sweep from the exact carry, backward sweep from zero
-            C y = lane == 0 ? yw : N::fma(f_ex, yw, bx);
+            C y = scan.forward_in(bx);
 #pragma unroll 2
             for (int i = 0; i < m; i++) {
                 const int q = i * kT + t;
@@ -462,23 +298,15 @@ __global__ void __launch_bounds__(kT, 1) propagate_cluster_kernel(Args P)
                 const int q = i * kT + t;
                 b = N::fms(gg[q], b, yv[q]);
             }
-#pragma unroll
-            for (int l = 0; l < 5; l++) {
-                const C dn = N::shdn(b, 1 << l);
-                if (lane + (1 << l) < 32) b = N::fma(b_lv[l], dn, b);
-            }
-            tot = N::bcast(b, 0);
-            if (lane <= rank) cluster.map_shared_rank(totB, lane)[g] = tot;
+            b = scan.backward_out(cluster, b);
             cluster.barrier_arrive();
             bx = N::shdn(b, 1);
             const C* ps = phs + ((int)(k / kPhSteps % 2) * kPhSteps + kp) * kPh;
             C ph = N::mul(N::mul(ps[lane >> 2], ps[kPhA + (lane & 3)]), ps[kPhA + kPhB + w]);
             const C zc = ps[kPh - 1];
             cluster.barrier_wait();
-            C uw = N::zero();
-            for (int q = 0; q < KB; q++) uw = N::fma(wtB[w * NW + q], totB[g + 1 + q], uw);
             // ---- backward sweep from the exact carry, CN update, phase e^{+i F dt x}, observables
-            C u = lane == 31 ? uw : N::fma(b_ex, uw, bx);
+            C u = scan.backward_in(bx);
             typename N::Acc acc;
 #pragma unroll 2
             for (int i = m - 1; i >= 0; i--) {
@@ -594,10 +422,10 @@ namespace mma {
 // grids of 601 to 8001 sites (us per step, measured / model):
 //   one CTA    FP64   601 sites  24.3 / 24.3    8001 sites  108.8 / 108.7   256 x 4001 sites  125 / 124
 //              df64   601 sites   7.8 /  7.8    8001 sites   35.1 /  35.1   304 x 8001 sites  58.8 / 58.9
-//   cluster    FP64  8001 sites  NC = 4  29.0 / 28.9   8  17.3 / 17.3   16  11.7 / 11.5;  256 x 4001, NC = 2  115 / 116
+//   cluster    FP64  8001 sites  NC = 4  29.0 / 28.8   8  17.3 / 17.2   16  11.7 / 11.4;  256 x 4001, NC = 2  115 / 115
 //              df64  8001 sites  NC = 4  10.1 / 10.1   8   6.9 /  7.2   16   5.6 /  5.7
-// FP64 is bound by the FP64 pipe, so CTAs that share an SM add their times (all but the barriers'); the
-// float-float form by latency, so a second CTA costs about two thirds of the first.
+// A second CTA on an SM costs FP64 its pipe time (16.1 us a wave measured at m = 4, 17.4 modelled) and
+// the float-float form, bound by latency, about two thirds of the first.
 namespace {
 double one_cta_us(int m256, int precision, int n_inst, int sms)
 {
@@ -608,7 +436,7 @@ double one_cta_us(int m256, int precision, int n_inst, int sms)
 }
 double cluster_us(int m, int precision, int waves, int per_sm)
 {
-    if (precision != 2) return waves * (2.4 + per_sm * (3.3 + 1.45 * m));
+    if (precision != 2) return waves * (4.0 + 0.35 * m + per_sm * (1.6 + 1.1 * m));
     return waves * (4.2 + 0.37 * m) * (1.0 + 0.65 * (per_sm - 1));
 }
 }  // namespace

@@ -113,3 +113,35 @@ def test_cluster_uneven_batch_with_too_wide_grid(gpu_lib):
         for k in SERIES:
             assert rel_l2(outs[1].series(i)[k].cpu().numpy(), outs[0].series(i)[k].cpu().numpy()) < 1e-10
     assert torch.isnan(outs[1].series(2)["sourceterm"]).all()
+
+
+class _OneCta:
+    """The library with a default of one CTA: batches of two then keep the one-CTA kernels."""
+
+    def __init__(self, lib):
+        self._lib = lib
+
+    def __getattr__(self, name):
+        return (lambda *a: 1) if name == "mma_tdse_default_ctas" else getattr(self._lib, name)
+
+
+@pytest.mark.parametrize("num_r, dx, K", [(4, 0.4, 8), (127, 0.3, 7), (128, 0.3, 1), (640, 0.2, 64), (2047, 0.2, 9),
+                                          (8000, 0.1, 32), (1500, 0.02, 16)])
+def test_adjoint_cluster_matches_one_cta_kernel(gpu_lib, monkeypatch, num_r, dx, K):
+    """The cluster form of the adjoint sweep (segments that end inside a batch of phases or of collected
+    sums, chunks of one site, threads without sites): 1e-10, as for the propagation."""
+    import mma_gb300.tdse_adjoint as ta
+    from mma_gb300.tdse_batch import TDSEGrids
+
+    t, E = _field(75)
+    fields = torch.tensor(np.stack([E, 0.7 * E[::-1].copy()]), device="cuda")
+    grids = TDSEGrids([dict(num_r=num_r, dx=dx, trg_a=A_CONFIG)], dt=0.25, adjoint=True)
+    band = (0.2, 1.5)
+    L, g = ta.yield_and_grad(grids, fields, 0.25, band, ckpt_every=K)
+    lib = ta._adj_sig()
+    monkeypatch.setattr(ta, "_adj_sig", lambda: _OneCta(lib))
+    L1, g1 = ta.yield_and_grad(grids, fields, 0.25, band, ckpt_every=K)
+    torch.cuda.synchronize()
+    assert rel_l2(L.cpu().numpy(), L1.cpu().numpy()) < 1e-10
+    for i in range(2):
+        assert rel_l2(g[i].cpu().numpy(), g1[i].cpu().numpy()) < 1e-10, i
