@@ -3,8 +3,8 @@
 //     window_analysis): for every energy E_i two complex Numerov-tridiagonal solves,
 //       (M2 (E_i - dE - i dE - V) - K) u1 = M2 psi,   (M2 (E_i + dE + i dE - V) - K) u2 = M2 u1,
 //       PES_i = dx dE^4 sum_j |u2_j|^2,
-//     one thread per energy, each a serial FP64 Thomas sweep (tridiag.c:26-70, 251-274) with its
-//     elimination factors interleaved across energies so that a warp's loads coalesce;
+//     by two threads per energy that eliminate from both ends, or a warp per energy (tridiag.c:26-70,
+//     251-274), in FP64 and with the elimination factors interleaved so that a warp's loads coalesce;
 //   * the Gabor transform (tools_fftw3.c:158-213, GaborTransform): for every window centre
 //     t_w = t_min + w (t_max - t_min)/N_G the signal times exp(-((t_j - t_w)/a)^2), a real DFT
 //     (this library's own, dft.cu, batched over windows and signals) and dt/sqrt(2 pi) |DFT_k| for
@@ -25,118 +25,313 @@ namespace an {
 
 constexpr double kPi = 3.14159265358979323846;
 
-// Energy-independent tables of the photoelectron spectrum: x_k = k dx - xmax with
-// xmax = 0.5 num_r dx (tools.c:231, 246), V(x_k) = -1/sqrt(a^2 + x^2) (tools.c:91-95) kept as
-// V/12 (n + 1 entries: the reference reads x[num_r + 1] for an unused super-diagonal of the
-// last row), and the right-hand side of the first solve, M2 psi = (10 psi_j + psi_{j-1} +
-// psi_{j+1})/12 (tridiag.c:261-268), which is the same for every energy.
-__global__ void pes_tables(int64_t n, int num_r, double dx, double a, const double* psi, double* V12, cd* rhs0)
-{
-    const double xmax = __dmul_rn(__dmul_rn(0.5, (double)num_r), dx);
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k <= n; k += (int64_t)gridDim.x * blockDim.x) {
-        const double x = __dsub_rn(__dmul_rn((double)k, dx), xmax);
-        V12[k] = (-1.0 / sqrt(a * a + x * x)) / 12.;
-        if (k < n) {
-            const cd pc{psi[2 * k], psi[2 * k + 1]};
-            const cd pm = k > 0 ? cd{psi[2 * k - 2], psi[2 * k - 1]} : cd{0.0, 0.0};
-            const cd pn = k + 1 < n ? cd{psi[2 * k + 2], psi[2 * k + 3]} : cd{0.0, 0.0};
-            rhs0[k] = cd{10 * pc.re / 12. + (pn.re + pm.re) / 12., 10 * pc.im / 12. + (pn.im + pm.im) / 12.};
-        }
-    }
-}
-
+// Both kernels below share the row arithmetic.  Row j of (M2 (Es -/+ i dE - V) - K) couples u_{j-1},
+// u_j, u_{j+1} by w_{j-1}, b_j, w_{j+1} (tools.c:257-275):
+//   w_j = (Es - V_j)/12 + 0.5/dx^2 -/+ i dE/12,  b_j = 10 (Es - V_j)/12 - 1/dx^2 -/+ i 10 dE/12,
+// and the elimination in either direction is gamma_j = w_j / beta_p, beta_j = b_j - w_p gamma_j,
+// y_j = (r_j - w_p y_p)/beta_j with p the row before, then u_p = y_p - gamma_j u_j backwards
+// (tridiag.c:26-70), with one reciprocal of |beta|^2 per row.
 struct PesArgs {
-    int64_t n;        // rows = num_r + 1
+    int64_t n;  // rows = num_r + 1
     double dx, dE, Estep, E_start;
-    int num_E, e0, chunk;
-    const double* V12;  // [n + 1]  V / 12
-    const cd* rhs0;     // [n]      M2 psi
-    cd* gam;            // [n][chunk]
-    cd* u;              // [n][chunk]
-    double* pes;        // [num_E]
+    int num_E, e0, count;  // energies e0 .. e0 + count - 1 of num_E
+    const double* V12;     // V / 12
+    const cd* rhs0;        // M2 psi
+    double* pes;           // [num_E]
 };
 
-// One Numerov-tridiagonal solve for the energy of this thread (sg = -1: first window, +1:
-// second).  Rows of (M2 (Es -/+ i dE - V) - K): diagonal 10 (Es - V_j)/12 - 1/dx^2 -/+ i 10 dE/12,
-// sub-diagonal of row j (Es - V_{j-1})/12 + 0.5/dx^2 -/+ i dE/12, super-diagonal of row j-1
-// (Es - V_j)/12 + 0.5/dx^2 -/+ i dE/12 (tools.c:257-275).  The right-hand side is M2 psi (first
-// solve) or M2 u1 formed from the first solve's result, which the sweep overwrites row by row
-// after reading it.  The Thomas recurrence is that of tridiag.c:26-70 with one reciprocal of
-// |beta|^2 per row; Es/12 and V/12 are formed once, so the rows need no divisions.
-__device__ __forceinline__ void pes_solve(const PesArgs& A, int e, double E, double sg, bool rhs_from_u,
-                                          double* norm_out)
+// The rows of one energy and window (sg = -1: first, +1: second).  Energy and potential are combined
+// before the 1/dx^2 terms, as in the reference: with Es/12 + 0.5/dx^2 formed once, its rounding is the
+// same in every row, an energy shift that the 1/dE of the window amplifies (7 times the error).
+struct Rows {
+    double e12, e10, diag, off, wi, bi;
+    __device__ Rows(const PesArgs& A, int ie, double sg)
+    {
+        const double Es = (A.E_start + A.Estep * ie) + sg * A.dE, s = sg < 0 ? -1.0 : 1.0;
+        e12 = Es / 12.;
+        e10 = 10 * Es / 12.;
+        diag = 1. / (A.dx * A.dx);
+        off = -0.5 / (A.dx * A.dx);
+        wi = s * (A.dE / 12);
+        bi = s * (10 * A.dE / 12);
+    }
+    __device__ cd w(double v12) const { return cd{(e12 - v12) - off, wi}; }
+    __device__ cd b(double v12) const { return cd{fma(-10.0, v12, e10) - diag, bi}; }
+};
+
+__device__ __forceinline__ cd cinv(cd b)
 {
-    const int64_t n = A.n, C = A.chunk;
-    const double Es = E + sg * A.dE;  // E_start + Estep i -/+ dE
-    const double e12 = Es / 12., e10 = 10 * Es / 12.;
-    const double diag = 1. / (A.dx * A.dx), off = -0.5 / (A.dx * A.dx);
-    const double im_d = (sg < 0 ? -1.0 : 1.0) * (10 * A.dE / 12), im_o = (sg < 0 ? -1.0 : 1.0) * (A.dE / 12);
+    const double s = 1.0 / fma(b.re, b.re, b.im * b.im);
+    return cd{b.re * s, -b.im * s};
+}
+__device__ __forceinline__ cd ldro(const cd* p)  // read-only for the whole launch
+{
+    const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+    return cd{v.x, v.y};
+}
+// M2 u of a row
+__device__ __forceinline__ cd m2(cd m, cd c, cd p)
+{
     constexpr double k12 = 1.0 / 12.;
-    cd pm{0.0, 0.0}, pc{0.0, 0.0}, pn{0.0, 0.0};
-    if (rhs_from_u) {
-        pc = A.u[e];
-        pn = (n > 1) ? A.u[C + e] : cd{0.0, 0.0};
-    }
-    auto rhs = [&](int64_t j) -> cd {
-        if (!rhs_from_u) return A.rhs0[j];
-        return cd{(10 * pc.re + (pn.re + pm.re)) * k12, (10 * pc.im + (pn.im + pm.im)) * k12};
-    };
-    // row 0
-    cd r = rhs(0);
-    double v12 = A.V12[0];
-    double b_re = (e10 - 10 * v12) - diag, b_im = im_d;
-    double bet_re = b_re, bet_im = b_im;
-    double inv = 1.0 / (bet_re * bet_re + bet_im * bet_im);
-    cd uprev{(r.re * b_re + r.im * b_im) * inv, (r.im * b_re - r.re * b_im) * inv};
-    A.u[e] = uprev;
-    for (int64_t j = 1; j < n; j++) {
-        if (rhs_from_u) {
-            pm = pc;
-            pc = pn;
-            pn = (j + 1 < n) ? A.u[(j + 1) * C + e] : cd{0.0, 0.0};
-        }
-        r = rhs(j);
-        const double v12j = A.V12[j];
-        const double a_re = (e12 - v12) - off, a_im = im_o;   // dinf[j-1]
-        const double c_re = (e12 - v12j) - off, c_im = im_o;  // dsup[j-1]
-        const double g_re = (c_re * bet_re + c_im * bet_im) * inv;
-        const double g_im = (c_im * bet_re - c_re * bet_im) * inv;
-        A.gam[j * C + e] = cd{g_re, g_im};
-        b_re = (e10 - 10 * v12j) - diag;
-        bet_re = b_re - (a_re * g_re - a_im * g_im);
-        bet_im = b_im - (a_im * g_re + a_re * g_im);
-        inv = 1.0 / (bet_re * bet_re + bet_im * bet_im);
-        const double t_re = r.re - a_re * uprev.re + a_im * uprev.im;
-        const double t_im = r.im - a_re * uprev.im - a_im * uprev.re;
-        uprev = cd{(t_re * bet_re + t_im * bet_im) * inv, (-t_re * bet_im + t_im * bet_re) * inv};
-        A.u[j * C + e] = uprev;  // the rhs of row j+1 already holds u1_j (pc) and u1_{j+1} (pn)
-        v12 = v12j;
-    }
-    // back substitution (tridiag.c:62-66)
-    cd unext = uprev;
-    double nrm = unext.re * unext.re + unext.im * unext.im;
-    for (int64_t j = n - 2; j >= 0; j--) {
-        const cd g = A.gam[(j + 1) * C + e];
-        cd uj = A.u[j * C + e];
-        uj.re -= g.re * unext.re - g.im * unext.im;
-        uj.im -= g.re * unext.im + g.im * unext.re;
-        A.u[j * C + e] = uj;
-        nrm += uj.re * uj.re + uj.im * uj.im;
-        unext = uj;
-    }
-    *norm_out = nrm;
+    return cd{fma(10.0, c.re, p.re + m.re) * k12, fma(10.0, c.im, p.im + m.im) * k12};
 }
 
-__global__ void __launch_bounds__(64) pes_kernel(PesArgs A)
+// fn(k, ld(k)) for k = 0 .. cnt - 1, the loads of a block of B one block ahead of their use: a row of a
+// substitution is six operations, about 400 cycles of a pipe that one warp feeds, and its loads take
+// a thousand (a wave of pairs 15.4 ms without this, 12.4 with)
+template <int B, typename Ld, typename Fn>
+__device__ __forceinline__ void piped(int64_t cnt, Ld ld, Fn fn)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ie = A.e0 + e;
-    if (e >= A.chunk || ie >= A.num_E) return;
-    const double E = A.E_start + A.Estep * ie;
-    double nrm;
-    pes_solve(A, e, E, -1.0, false, &nrm);
-    pes_solve(A, e, E, +1.0, true, &nrm);
-    A.pes[ie] = nrm * A.dx * pow(A.dE, 4.);
+    typedef decltype(ld((int64_t)0)) V;
+    V cur[B], nxt[B];
+#pragma unroll
+    for (int q = 0; q < B; q++)
+        if (q < cnt) cur[q] = ld(q);
+    for (int64_t k = 0; k < cnt; k += B) {
+#pragma unroll
+        for (int q = 0; q < B; q++)
+            if (k + B + q < cnt) nxt[q] = ld(k + B + q);
+#pragma unroll
+        for (int q = 0; q < B; q++)
+            if (k + q < cnt) fn(k + q, cur[q]);
+#pragma unroll
+        for (int q = 0; q < B; q++) cur[q] = nxt[q];
+    }
+}
+struct Two {
+    cd g, y;
+};
+struct Three {
+    cd g, y, f;
+};
+
+// Energy-independent tables: x_k = k dx - xmax with xmax = 0.5 num_r dx (tools.c:231, 246), V(x_k) =
+// -1/sqrt(a^2 + x^2) (tools.c:91-95) kept as V/12, and the right-hand side of the first solve, M2 psi =
+// (10 psi_j + psi_{j-1} + psi_{j+1})/12 (tridiag.c:261-268), the same for every energy; in natural order
+// and, rows beyond the grid zero, with row j = s m + i at [i][s] for the warp kernel (s < 32).
+__global__ void pes_tables(int64_t n, int64_t m, int num_r, double dx, double a, const double* psi, double* V12,
+                           cd* rhs0, double* V12t, cd* rhs0t)
+{
+    const double xmax = __dmul_rn(__dmul_rn(0.5, (double)num_r), dx);
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < 32 * m; k += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t q = k % m * 32 + k / m;
+        if (k >= n) {
+            V12t[q] = 0.0;
+            rhs0t[q] = cd{0.0, 0.0};
+            continue;
+        }
+        const double x = __dsub_rn(__dmul_rn((double)k, dx), xmax);
+        const double v = (-1.0 / sqrt(a * a + x * x)) / 12.;
+        const cd pc{psi[2 * k], psi[2 * k + 1]};
+        const cd pm = k > 0 ? cd{psi[2 * k - 2], psi[2 * k - 1]} : cd{0.0, 0.0};
+        const cd pn = k + 1 < n ? cd{psi[2 * k + 2], psi[2 * k + 3]} : cd{0.0, 0.0};
+        const cd r{10 * pc.re / 12. + (pn.re + pm.re) / 12., 10 * pc.im / 12. + (pn.im + pm.im) / 12.};
+        V12[k] = V12t[q] = v;
+        rhs0[k] = rhs0t[q] = r;
+    }
+}
+
+// ------------------------------------------------------------------------ two threads per energy
+// Elimination from both ends towards the middle and substitution outwards again: the operations of one
+// Thomas sweep at half its length, on twice the threads.  A CTA takes 64 energies; its four warps (two
+// groups of energies, two sides) sit on the SM's four sub-partitions, whose FP64 pipes they fill: a full
+// wave is 64 energies an SM.  One thread per energy left two of the four pipes of each SM idle.
+struct PesPair {
+    PesArgs A;
+    cd* gam;  // [n][stride]
+    cd* u;    // [n][stride]
+    int64_t stride;
+};
+
+__device__ __forceinline__ void pes_pair(const PesPair& Q)
+{
+    const PesArgs& A = Q.A;
+    __shared__ cd s_y[2][64], s_g[2][64];
+    __shared__ double s_n[64];
+    const int w = threadIdx.x >> 5, side = w >> 1, el = (w & 1) * 32 + (threadIdx.x & 31);
+    int e = blockIdx.x * 64 + el;
+    const bool live = e < A.count;
+    if (!live) e = A.count - 1;  // an idle lane repeats the last energy into no output and no buffer
+    const int64_t n = A.n, h = n / 2, C = Q.stride;
+    const int64_t d = side ? -1 : 1, first = side ? n - 1 : 0, cnt = side ? n - h : h;
+    cd* const gam = Q.gam + e;
+    cd* const u = Q.u + e;
+    cd mine{0.0, 0.0}, other{0.0, 0.0};  // the solution at the last row of this side and of the other
+    double nrm = 0.0;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+        const Rows R(A, A.e0 + e, pass ? 1.0 : -1.0);
+        cd pm{0.0, 0.0}, pc{0.0, 0.0}, pn{0.0, 0.0};
+        if (pass) {
+            pc = cnt > 1 ? u[first * C] : mine;
+            pn = cnt > 2 ? u[(first + d) * C] : cnt > 1 ? mine : other;
+        }
+        cd wp{0.0, 0.0}, ibeta{0.0, 0.0}, y{0.0, 0.0};
+#pragma unroll 2
+        for (int64_t i = 0; i < cnt; i++) {
+            const int64_t j = first + d * i;
+            const double v = __ldg(A.V12 + j);
+            const cd wj = R.w(v);
+            cd r;
+            if (pass) {
+                r = m2(pm, pc, pn);
+                pm = pc;
+                pc = pn;
+                pn = i + 3 < cnt ? u[(j + 2 * d) * C] : i + 3 == cnt ? mine : other;
+            } else {
+                r = ldro(A.rhs0 + j);
+            }
+            const cd g = cmul(wj, ibeta);
+            ibeta = cinv(cfms(wp, g, R.b(v)));
+            y = cmul(cfms(wp, y, r), ibeta);
+            wp = wj;
+            if (live) {
+                gam[j * C] = g;
+                u[j * C] = y;
+            }
+        }
+        // the two middle rows: u_a = y_a - g_a u_b, u_b = y_b - g_b u_a
+        s_y[side][el] = y;
+        s_g[side][el] = cmul(R.w(A.V12[side ? h - 1 : h]), ibeta);
+        __syncthreads();
+        const cd yo = s_y[1 - side][el], go = s_g[1 - side][el], gm = s_g[side][el];
+        const cd det = cfms(gm, go, cd{1.0, 0.0});
+        mine = cmul(cfms(gm, yo, y), cinv(det));
+        other = cfms(go, mine, yo);
+        __syncthreads();
+        // substitution outwards; the middle row's value stays in a register (the second pass reads it there)
+        cd un = mine;
+        nrm = un.re * un.re + un.im * un.im;
+        const int64_t top = first + d * (cnt - 2);  // row of k = 0
+        piped<4>(
+            cnt - 1, [&](int64_t k) { return Two{gam[(top - d * k + d) * C], u[(top - d * k) * C]}; },
+            [&](int64_t k, const Two& v) {
+                un = cfms(v.g, un, v.y);
+                if (live && pass == 0) u[(top - d * k) * C] = un;
+                nrm = fma(un.re, un.re, fma(un.im, un.im, nrm));
+            });
+    }
+    if (side) s_n[el] = nrm;
+    __syncthreads();
+    if (!side && live) A.pes[A.e0 + e] = (nrm + s_n[el]) * A.dx * pow(A.dE, 4.);
+}
+
+// ------------------------------------------------------------------------ one warp per energy
+// Lane s owns rows s m .. s m + m - 1 and eliminates them from its first row on, carrying the dependence
+// f_j on the row before the chunk (u_j = y_j + f_j u_L - gamma_{j+1} u_{j+1}).  A backward pass without
+// stores expresses the chunk's first value by u_L and its last value z; the 32 last values then satisfy a
+// tridiagonal system across the lanes (parallel cyclic reduction, five levels), and a second backward
+// pass gives u.  About 66 FP64 operations a row and solve against 42 of the pair kernel, but 1/32 of its
+// chain: few energies, and what full waves of the pair kernel leave over, run here.
+struct PesWarp {
+    PesArgs A;
+    int64_t m;
+    cd* buf;  // per warp: gamma, y (then u), f, each [m][32]
+};
+
+__device__ __forceinline__ void pes_warp(const PesWarp& Q, int block, int blocks)
+{
+    const PesArgs& A = Q.A;
+    const int lane = threadIdx.x & 31, slot = block * 4 + (threadIdx.x >> 5), slots = blocks * 4;
+    const int64_t m = Q.m, n = A.n;
+    cd* const gam = Q.buf + (int64_t)slot * 96 * m + lane;
+    cd* const yb = gam + 32 * m;
+    cd* const fb = yb + 32 * m;
+    const int64_t a = lane * m, left = n - a;
+    const int64_t cnt = left < 0 ? 0 : left < m ? left : m;  // rows of this lane
+    const cd zero{0.0, 0.0};
+    auto from = [](cd v, int l) { return cd{shfl_idx(v.re, l), shfl_idx(v.im, l)}; };
+    for (int e = slot; e < A.count; e += slots) {
+        double nrm = 0.0;
+        cd uL = zero, uR = zero;  // solution of the first window beside the chunk
+#pragma unroll 1
+        for (int pass = 0; pass < 2; pass++) {
+            const Rows R(A, A.e0 + e, pass ? 1.0 : -1.0);
+            cd wp = lane > 0 && cnt > 0 ? R.w(A.V12[(m - 1) * 32 + lane - 1]) : zero;  // w of the row before the chunk
+            cd ibeta = zero, y = zero, f = cd{1.0, 0.0};
+            cd pm = uL, pc = pass ? yb[0] : zero, pn = zero;
+            for (int64_t i = 0; i < cnt; i++) {
+                const double v = __ldg(A.V12 + i * 32 + lane);
+                const cd wj = R.w(v);
+                cd r;
+                if (pass) {
+                    pn = i + 1 < cnt ? yb[(i + 1) * 32] : uR;
+                    r = m2(pm, pc, pn);
+                    pm = pc;
+                    pc = pn;
+                } else {
+                    r = ldro(A.rhs0 + i * 32 + lane);
+                }
+                const cd g = cmul(wj, ibeta);  // 0 in the chunk's first row: the elimination starts afresh
+                const cd beta = i > 0 ? cfms(wp, g, R.b(v)) : R.b(v);
+                ibeta = cinv(beta);
+                const cd hq = cmul(wp, ibeta);
+                y = cfms(hq, y, cmul(r, ibeta));
+                f = cfms(hq, f, zero);
+                gam[i * 32] = g;
+                yb[i * 32] = y;
+                fb[i * 32] = f;
+                wp = wj;
+            }
+            // u_first = Y + F u_L + H z
+            cd Y = zero, F = zero, H = cd{1.0, 0.0};
+            auto row = [&](int64_t k) {
+                const int64_t i = cnt - 2 - k;
+                return Three{gam[(i + 1) * 32], yb[i * 32], fb[i * 32]};
+            };
+            piped<2>(cnt - 1, row, [&](int64_t, const Three& v) {
+                Y = cfms(v.g, Y, v.y);
+                F = cfms(v.g, F, v.f);
+                H = cfms(v.g, H, zero);
+            });
+            // z_s (1 + g F') = (y - g Y') + f z_{s-1} - g H' z_{s+1}, primes: the next lane's chunk
+            const bool next = lane < 31 && a + m < n;
+            const cd gb = next ? cmul(R.w(A.V12[lane + 1]), ibeta) : zero;
+            const cd Yn = from(Y, lane + 1 < 32 ? lane + 1 : 31), Fn = from(F, lane + 1 < 32 ? lane + 1 : 31),
+                     Hn = from(H, lane + 1 < 32 ? lane + 1 : 31);
+            cd iq = cinv(cfma(gb, Fn, cd{1.0, 0.0}));
+            if (cnt == 0) y = f = zero;
+            cd Rz = cmul(cfms(gb, Yn, y), iq), Az = lane > 0 ? cmul(f, iq) : zero, Cz = cmul(cfms(gb, Hn, zero), iq);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int lo = lane - d < 0 ? 0 : lane - d, hi = lane + d > 31 ? 31 : lane + d;
+                const cd Rm = from(Rz, lo), Am = from(Az, lo), Cm = from(Cz, lo);
+                const cd Rp = from(Rz, hi), Ap = from(Az, hi), Cp = from(Cz, hi);
+                iq = cinv(cfms(Cz, Ap, cfms(Az, Cm, cd{1.0, 0.0})));
+                Rz = cmul(cfma(Cz, Rp, cfma(Az, Rm, Rz)), iq);
+                Az = cmul(cmul(Az, Am), iq);
+                Cz = cmul(cmul(Cz, Cp), iq);
+                if (lane < 2 * d) Az = zero;
+                if (lane + 2 * d > 31) Cz = zero;
+            }
+            const cd z = Rz, zl = from(z, lane > 0 ? lane - 1 : 0);
+            const cd vL = lane > 0 ? zl : zero;
+            cd u = z;
+            if (cnt > 0) {
+                nrm = u.re * u.re + u.im * u.im;
+                if (pass == 0) yb[(cnt - 1) * 32] = u;
+            }
+            piped<2>(cnt - 1, row, [&](int64_t k, const Three& v) {
+                u = cfms(v.g, u, cfma(v.f, vL, v.y));
+                if (pass == 0) yb[(cnt - 2 - k) * 32] = u;
+                nrm = fma(u.re, u.re, fma(u.im, u.im, nrm));
+            });
+            uL = vL;  // and the next lane's first value
+            const cd un = from(u, lane + 1 < 32 ? lane + 1 : 31);
+            uR = next ? un : zero;
+        }
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) nrm += shfl_xor(nrm, d);
+        if (lane == 0) A.pes[A.e0 + e] = nrm * A.dx * pow(A.dE, 4.);
+    }
+}
+
+// A wave of pairs (the first `pairs` CTAs) and the energies beyond it a warp each (the others), which
+// share the SMs: the pairs' one warp per pipe leaves a quarter of its cycles free.
+__global__ void __launch_bounds__(128) pes_kernel(PesPair Q, int pairs, PesWarp W)
+{
+    if ((int)blockIdx.x < pairs) pes_pair(Q);
+    else pes_warp(W, blockIdx.x - pairs, gridDim.x - pairs);
 }
 
 // Gabor windows exp(-(ia (j dt - (t_min + w dt_G)))^2) (tools_fftw3.c:180-196, ia = 1/a), the
@@ -184,37 +379,85 @@ using namespace mma;
 namespace {
 // scratch: V/12 [n + 1] | M2 psi [n] | gam [n][chunk] | u [n][chunk]
 size_t pes_fixed(size_t n) { return (sizeof(double) * (n + 1) + 255) / 256 * 256 + (sizeof(cd) * n + 255) / 256 * 256; }
+
+int pes_sms()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
+}
 }  // namespace
 
 extern "C" size_t mma_tdse_pes_scratch_bytes(int num_r, int chunk)
 {
     if (num_r < 1 || chunk < 1) return 0;
-    const size_t n = (size_t)num_r + 1;
-    return pes_fixed(n) + 2 * sizeof(cd) * n * (size_t)chunk;
+    const size_t n = (size_t)num_r + 1, m = (n + 31) / 32;
+    // the pairs' two arrays of `chunk` energies, then gamma, y and f of the energies that a warp each
+    // takes: those beyond full waves of pairs, as many as run at once (16 warps an SM)
+    const size_t wave = 64 * 152, rest = (size_t)chunk % wave * 5 > wave * 3 ? 0 : (size_t)chunk % wave;
+    const size_t warps = ((size_t)chunk < wave ? (size_t)chunk : rest) + 3;
+    return pes_fixed(n) + 32 * m * 24 + 512 + 2 * sizeof(cd) * n * ((size_t)chunk - rest) +
+           48 * 32 * m * ((warps < 16 * 152 ? warps : 16 * 152) / 4 * 4);
 }
 
 extern "C" int mma_tdse_pes(const double* psi, int num_r, double dx, double trg_a, int num_E, double dE, double Estep,
                             double E_start, double* pes, void* scratch, size_t scratch_bytes, void* stream)
 {
     if (!psi || !pes || !scratch || num_r < 1 || num_E < 1 || !(dx > 0.0)) return MMA_ERR_ARG;
-    const int64_t n = (int64_t)num_r + 1;
+    const int64_t n = (int64_t)num_r + 1, m = (n + 31) / 32;
     const size_t fixed = pes_fixed((size_t)n);
     if (scratch_bytes < fixed + 2 * sizeof(cd) * (size_t)n) return MMA_ERR_ARG;
-    int64_t chunk = (int64_t)((scratch_bytes - fixed) / (2 * sizeof(cd) * (size_t)n));
-    if (chunk > num_E) chunk = num_E;
     cudaStream_t st = (cudaStream_t)stream;
     char* sc = static_cast<char*>(scratch);
     double* V12 = reinterpret_cast<double*>(sc);
     cd* rhs0 = reinterpret_cast<cd*>(sc + (sizeof(double) * (size_t)(n + 1) + 255) / 256 * 256);
-    cd* gam = reinterpret_cast<cd*>(sc + fixed);
-    cd* u = gam + (size_t)n * chunk;
-    an::pes_tables<<<an::grid_for(n + 1), 256, 0, st>>>(n, num_r, dx, trg_a, psi, V12, rhs0);
-    for (int e0 = 0; e0 < num_E; e0 += (int)chunk) {
-        an::PesArgs A{n, dx, dE, Estep, E_start, num_E, e0, (int)chunk, V12, rhs0, gam, u, pes};
-        const int cnt = (int)((num_E - e0 < chunk) ? num_E - e0 : chunk);
-        an::pes_kernel<<<(cnt + 63) / 64, 64, 0, st>>>(A);  // small blocks: few energies still reach every SM
+    // behind the fixed tables: the warp kernel's tables, then either kernel's buffers
+    const size_t tabs = ((size_t)(32 * m) * 24 + 255) / 256 * 256, one = sizeof(cd) * 96 * (size_t)m;
+    char* rest = sc + fixed;
+    size_t room = scratch_bytes - fixed;
+    void* own = nullptr;
+    if (room < tabs + 4 * one) {  // a workspace of the least size the call takes: a few warps' worth of its own
+        room = tabs + 16 * one;
+        if (cudaMallocAsync(&own, room, st) != cudaSuccess) return MMA_ERR_CUDA;
+        rest = static_cast<char*>(own);
     }
-    return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+    cd* rhs0t = reinterpret_cast<cd*>(rest);
+    double* V12t = reinterpret_cast<double*>(rhs0t + 32 * m);
+    cd* buf = reinterpret_cast<cd*>(rest + tabs);
+    room -= tabs;
+    an::pes_tables<<<an::grid_for(32 * m), 256, 0, st>>>(n, m, num_r, dx, trg_a, psi, V12, rhs0, V12t, rhs0t);
+    // full waves of pairs (64 energies an SM), the rest a warp each where that is less than another wave:
+    // 66 operations a row against 40 with several warps a pipe, so up to about 0.6 of one.  8001 rows: a
+    // wave of pairs 13.0 ms (one thread an energy, all 10000: 34.2 ms; 13.9 with the rest), 5000 energies a
+    // warp each 11.0 ms, 50 energies 1.46 ms (29.0 ms).
+    const int sms = pes_sms(), wave = 64 * sms;
+    an::PesArgs A{n, dx, dE, Estep, E_start, num_E, 0, 0, V12, rhs0, pes};
+    for (int done = 0; done < num_E;) {
+        const int left = num_E - done;
+        int np = left * (int64_t)5 > wave * (int64_t)3 && n >= 4 ? (left < wave ? left : wave) : 0;
+        if (room < 2 * sizeof(cd) * (size_t)n * np) np = 0;
+        an::PesPair Q{A, buf, buf + (size_t)n * np, np};
+        Q.A.e0 = done;
+        Q.A.count = np;
+        done += np;
+        const size_t used = 2 * sizeof(cd) * (size_t)n * np;
+        int nw = num_E - done;
+        if (np > 0 && (nw * (int64_t)5 > wave * (int64_t)3 || room < used + 4 * one)) nw = 0;  // the next launch's
+        int64_t blocks = (int64_t)((room - used) / (4 * one));
+        if (blocks > 4 * sms) blocks = 4 * sms;
+        if (blocks > (nw + 3) / 4) blocks = (nw + 3) / 4;
+        an::PesWarp W{A, m, buf + 2 * (size_t)n * np};
+        W.A.e0 = done;
+        W.A.count = nw;
+        W.A.V12 = V12t;
+        W.A.rhs0 = rhs0t;
+        done += nw;
+        const int pairs = (np + 63) / 64;
+        an::pes_kernel<<<(unsigned)(pairs + blocks), 128, 0, st>>>(Q, pairs, W);
+    }
+    const bool ok = cudaGetLastError() == cudaSuccess;
+    if (own && cudaFreeAsync(own, st) != cudaSuccess) return MMA_ERR_CUDA;
+    return ok ? MMA_OK : MMA_ERR_CUDA;
 }
 
 extern "C" size_t mma_gabor_scratch_bytes(int n_sig, int N, int N_G)
