@@ -83,6 +83,18 @@ size_t mma_hankel_fast_scratch_bytes(const mma_hankel_problem *p, const mma_hank
  * for all n_z planes; complex128 planes [slot][n_rho][n_omega], ff [n_rho][n_omega]). */
 int mma_hankel_ff_from_planes(const mma_hankel_problem *p, const double *zgrid, const int64_t *plane_slot,
                               const double *planes, double *ff, void *stream);
+/* Running z trapezoid of every plane (the cumulative results of Hankel_long): planes [n_z][n_rho]
+ * [n_omega] in the order of zgrid; running [n_z - 1][n_rho][n_omega] = the sums up to planes 1 .. n_z - 1,
+ * normalised = renorm [n_z - 1 rows read][n_omega] times them.  Either output may be NULL (renorm too,
+ * without normalised). */
+int mma_hankel_cumulative(const mma_hankel_problem *p, const double *zgrid, const double *planes,
+                          const double *renorm, double *normalised, double *running, void *stream);
+/* Pre-factor [n_z][n_omega] (complex) and renormalisation [n_z][n_omega] (or NULL) of a medium of
+ * constant pressure: pre = pressure exp(w ((z - z_last) absorption(w) + i z dispersion(w))), renorm =
+ * exp((z_last - z) w absorption(w)); dispersion and absorption [n_omega]. */
+int mma_hankel_uniform_pre_factor(int64_t n_z, int64_t n_omega, const double *zgrid, const double *ogrid,
+                                  const double *dispersion, const double *absorption, double pressure, double *pre,
+                                  double *renorm, void *stream);
 /* Stage 1 of mma_hankel_fast (the z contraction B_m): mode 1 (default) runs it on the CUDA cores
  * (FP32 FMAs, the streamed ring form); mode 0 runs it on the tensor cores where it applies -- 16
  * series terms, a complex64 source with rows on 16-byte boundaries (even n_r and strides),

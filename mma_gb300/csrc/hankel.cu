@@ -1057,6 +1057,106 @@ extern "C" int mma_hankel_ff_from_planes(const mma_hankel_problem* p, const doub
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }
 
+// ------------------------------------------------------------------------ cumulative results
+// The running z trapezoid of all planes (Hankel_transform.py:640-672): run_k = sum_{q <= k} 0.5 dz_q
+// (P_q + P_{q+1}) for k = 0 .. n_z - 2, and renorm_k(w) run_k.  One thread per (rho, w) walks the planes
+// once, the loads of the next eight in flight over the sums of this eight.  Bound by the FP64 pipe: six
+// operations an element at two lanes a cycle and SM, 330 us for 512 w x 256 rho x 255 planes against 160
+// us for its 1.07 GB; the steps' widths come from shared memory (formed per thread they are two more
+// operations: 589 us).  460 us, against 1210 us for the stack, sums, scan and product as passes.
+constexpr int kCumChunk = 1024;
+
+__global__ void __launch_bounds__(kThreads) cumulative_kernel(int64_t nz, int64_t n, int64_t no,
+                                                              const double* __restrict__ zg,
+                                                              const double2* __restrict__ planes,
+                                                              const double* __restrict__ renorm,
+                                                              double2* __restrict__ norm_out, double2* __restrict__ run_out)
+{
+    __shared__ double s_h[kCumChunk];
+    const int64_t e = blockIdx.x * (int64_t)kThreads + threadIdx.x, a = e < n ? e : 0, o = a % no;
+    const bool live = e < n;
+    constexpr int B = 8;
+    double2 p = planes[a], run = make_double2(0.0, 0.0);
+    for (int64_t c0 = 0; c0 + 1 < nz; c0 += kCumChunk) {
+        const int cnt = (int)(nz - 1 - c0 < kCumChunk ? nz - 1 - c0 : kCumChunk);
+        __syncthreads();
+        for (int q = threadIdx.x; q < cnt; q += kThreads) s_h[q] = 0.5 * (zg[c0 + q + 1] - zg[c0 + q]);
+        __syncthreads();
+        double2 x[B], xn[B];
+        double rn[B], rnn[B];
+        auto load = [&](int k, double2 (&v)[B], double (&r)[B]) {
+#pragma unroll
+            for (int q = 0; q < B; q++)
+                if (k + q < cnt) {
+                    v[q] = __ldcs(planes + (c0 + k + 1 + q) * n + a);
+                    r[q] = norm_out ? renorm[(c0 + k + q) * no + o] : 0.0;
+                }
+        };
+        load(0, x, rn);
+        for (int k = 0; k < cnt; k += B) {
+            load(k + B, xn, rnn);
+#pragma unroll
+            for (int q = 0; q < B; q++)
+                if (k + q < cnt) {
+                    const double h = s_h[k + q];
+                    run.x = fma(h, p.x + x[q].x, run.x);
+                    run.y = fma(h, p.y + x[q].y, run.y);
+                    p = x[q];
+                    const int64_t at = (c0 + k + q) * n + a;
+                    if (live && norm_out) __stcs(norm_out + at, make_double2(rn[q] * run.x, rn[q] * run.y));
+                    if (live && run_out) __stcs(run_out + at, run);
+                }
+#pragma unroll
+            for (int q = 0; q < B; q++) {
+                x[q] = xn[q];
+                rn[q] = rnn[q];
+            }
+        }
+    }
+}
+
+extern "C" int mma_hankel_cumulative(const mma_hankel_problem* p, const double* zgrid, const double* planes,
+                                     const double* renorm, double* normalised, double* running, void* stream)
+{
+    if (!valid(p) || p->n_z < 2 || !zgrid || !planes || (!normalised && !running) || (normalised && !renorm))
+        return MMA_ERR_ARG;
+    const int64_t n = p->n_rho * p->n_omega, b = (n + kThreads - 1) / kThreads;
+    if (b > INT32_MAX) return MMA_ERR_TOO_LARGE;
+    cumulative_kernel<<<(unsigned)b, kThreads, 0, (cudaStream_t)stream>>>(
+        p->n_z, n, p->n_omega, zgrid, reinterpret_cast<const double2*>(planes), renorm,
+        reinterpret_cast<double2*>(normalised), reinterpret_cast<double2*>(running));
+    return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+}
+
+// Pre-factor and renormalisation of a medium of constant pressure (Hankel_transform.py:405-448):
+// pre = p exp(w ((z - z_last) a(w) + i z d(w))), renorm = exp((z_last - z) w a(w)).
+__global__ void __launch_bounds__(kThreads) uniform_pre_factor_kernel(int64_t nz, int64_t no, const double* zg,
+                                                                      const double* og, const double* d, const double* a,
+                                                                      double pressure, double2* pre, double* renorm)
+{
+    const double zl = zg[nz - 1];
+    for (int64_t q = blockIdx.x * (int64_t)kThreads + threadIdx.x; q < nz * no; q += (int64_t)gridDim.x * kThreads) {
+        const int64_t o = q % no;
+        const double w = og[o], z = zg[q / no];
+        double sn, cs;
+        sincos(w * (z * d[o]), &sn, &cs);
+        const double f = exp(w * ((z - zl) * a[o]));
+        pre[q] = make_double2(pressure * (f * cs), pressure * (f * sn));
+        if (renorm) renorm[q] = exp((zl - z) * (w * a[o]));
+    }
+}
+
+extern "C" int mma_hankel_uniform_pre_factor(int64_t n_z, int64_t n_omega, const double* zgrid, const double* ogrid,
+                                             const double* dispersion, const double* absorption, double pressure,
+                                             double* pre, double* renorm, void* stream)
+{
+    if (n_z < 1 || n_omega < 1 || !zgrid || !ogrid || !dispersion || !absorption || !pre) return MMA_ERR_ARG;
+    const int64_t b = (n_z * n_omega + kThreads - 1) / kThreads;
+    uniform_pre_factor_kernel<<<(unsigned)(b < 4096 ? b : 4096), kThreads, 0, (cudaStream_t)stream>>>(
+        n_z, n_omega, zgrid, ogrid, dispersion, absorption, pressure, reinterpret_cast<double2*>(pre), renorm);
+    return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+}
+
 // A block of frequencies [n_z][w0:w1][n_r] copied between two sources laid out alike (host and
 // device, either direction): n_z rows of block_bytes, the rows plane_bytes apart on both sides.
 // One asynchronous 2-D copy on `stream`.

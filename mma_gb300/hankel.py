@@ -96,6 +96,11 @@ def _sig():
     lib.mma_hankel_copy_block.restype = c_int
     lib.mma_hankel_ff_from_planes.argtypes = [P, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
     lib.mma_hankel_ff_from_planes.restype = c_int
+    lib.mma_hankel_cumulative.argtypes = [P, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
+    lib.mma_hankel_cumulative.restype = c_int
+    lib.mma_hankel_uniform_pre_factor.argtypes = [c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_double,
+                                                  c_void_p, c_void_p, c_void_p]
+    lib.mma_hankel_uniform_pre_factor.restype = c_int
     lib.mma_hankel_fast_status.argtypes = [P, POINTER(FastPlan), c_void_p, c_void_p]
     lib.mma_hankel_fast_status.restype = c_int
     lib._mma_hankel_sig = True
@@ -371,6 +376,38 @@ def _radial_pre_factor(z, r, w, gas, pressure, absorption_tables, include_absorp
     return pre
 
 
+def _uniform_medium(w, gas, pressure, absorption_tables, include_absorption, dispersion_tables, include_dispersion,
+                    n_ir):
+    """Per-frequency dispersion and absorption factors of a medium of constant pressure (:405-448)."""
+    if include_dispersion:
+        disp = XUV_index.dispersion_function(w, pressure, gas + "_" + dispersion_tables, n_IR=n_ir)
+    else:
+        disp = (n_ir - 1.0) / C_LIGHT * np.ones_like(w)
+    if include_absorption:
+        absorb = (pressure / C_LIGHT) * XUV_index.beta_factor_ref(w, gas + "_" + absorption_tables)
+    else:
+        absorb = np.zeros_like(w)
+    return disp, absorb
+
+
+def _uniform_tables_on_device(z, w, dev, pressure, want_renorm, **medium):
+    """pre_factor_table of a medium of constant pressure, evaluated on the device: (pre [Nz, No]
+    complex128, renorm [Nz, No] float64 or None) as tensors; None for complex factors (a complex IR
+    index), which the host's table takes.  [255, 512] tables: 3.6 ms of numpy a call, 20 us here."""
+    disp, absorb = _uniform_medium(w, pressure=pressure, **medium)
+    if np.iscomplexobj(disp) or np.iscomplexobj(absorb):
+        return None
+    pre = torch.empty(len(z), len(w), dtype=torch.complex128, device=dev)
+    renorm = torch.empty(len(z), len(w), dtype=torch.float64, device=dev) if want_renorm else None
+    zd, wd, dd, ad = (_dev(a, dev) for a in (z, w, np.broadcast_to(disp, w.shape), np.broadcast_to(absorb, w.shape)))
+    _check(_sig().mma_hankel_uniform_pre_factor(len(z), len(w), zd.data_ptr(), wd.data_ptr(), dd.data_ptr(),
+                                                ad.data_ptr(), float(pressure), pre.data_ptr(),
+                                                None if renorm is None else renorm.data_ptr(),
+                                                ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)),
+           "mma_hankel_uniform_pre_factor")
+    return pre, renorm
+
+
 def pre_factor_table(zgrid, ogrid, preset_gas="vacuum", pressure=1.0, absorption_tables="Henke",
                      include_absorption=True, dispersion_tables="Henke", include_dispersion=True,
                      effective_IR_refrective_index=1.0, rgrid=None):
@@ -413,14 +450,9 @@ def pre_factor_table(zgrid, ogrid, preset_gas="vacuum", pressure=1.0, absorption
             pre[:, k1] = p_loc * np.exp(w[k1] * (disp + absf))
         renorm = np.exp(absw[-1][None, :] - absw)
         return pre, renorm
-    if include_dispersion:
-        disp = 1j * XUV_index.dispersion_function(w, pressure, preset_gas + "_" + dispersion_tables, n_IR=n_ir)
-    else:
-        disp = 1j * (n_ir - 1.0) / C_LIGHT * np.ones_like(w)
-    if include_absorption:
-        absorb = (pressure / C_LIGHT) * XUV_index.beta_factor_ref(w, preset_gas + "_" + absorption_tables)
-    else:
-        absorb = np.zeros_like(w)
+    disp, absorb = _uniform_medium(w, preset_gas, pressure, absorption_tables, include_absorption, dispersion_tables,
+                                   include_dispersion, n_ir)
+    disp = 1j * disp
     pre = pressure * np.exp(w[None, :] * (z[:, None] * disp[None, :] + (z[:, None] - z[-1]) * absorb[None, :]))
     renorm = np.exp((z[-1] - z[:, None]) * (w * absorb)[None, :])
     return pre, renorm
@@ -740,11 +772,21 @@ class Hankel_long:
             raise ValueError("Wrongly specified preset gas (or tables).")
         if store_cumulative_result and isinstance(pressure, dict) and "rgrid" in pressure:
             raise NotImplementedError("Renormalisation of the signal is not implemented for radially modulated density.")
-        pre, renorm = pre_factor_table(target.zgrid, target.ogrid, preset_gas, pressure, absorption_tables,
-                                       include_absorption, dispersion_tables, include_dispersion,
-                                       effective_IR_refrective_index, rgrid=target.rgrid)
         z = np.asarray(target.zgrid, dtype=np.float64)
         Nz = len(z)
+        tables = None
+        if target.source.is_cuda and isinstance(pressure, (int, float, np.integer, np.floating)) and Nz > 0:
+            tables = _uniform_tables_on_device(
+                z, np.asarray(target.ogrid, dtype=np.float64), target.source.device, pressure, store_cumulative_result,
+                gas=preset_gas, absorption_tables=absorption_tables, include_absorption=include_absorption,
+                dispersion_tables=dispersion_tables, include_dispersion=include_dispersion,
+                n_ir=effective_IR_refrective_index)
+        if tables is not None:
+            pre, renorm = tables
+        else:
+            pre, renorm = pre_factor_table(target.zgrid, target.ogrid, preset_gas, pressure, absorption_tables,
+                                           include_absorption, dispersion_tables, include_dispersion,
+                                           effective_IR_refrective_index, rgrid=target.rgrid)
         if Nz < 2:
             raise ValueError("Hankel_long needs at least two source planes")
         want = set()
@@ -761,15 +803,31 @@ class Hankel_long:
             self.entry_plane_transform = conv(planes[0])
             self.exit_plane_transform = conv(planes[Nz - 1])
         if cum:
-            P = torch.stack([planes[k] for k in range(Nz)])  # [Nz, Nrho, No]
-            dz = torch.as_tensor(np.diff(z), device=P.device, dtype=torch.float64)
-            contrib = 0.5 * dz[:, None, None] * (P[:-1] + P[1:])
-            run = torch.cumsum(contrib, dim=0)  # running z-trapezoid after planes 1..Nz-1
+            norm, run = _cumulative(z, [planes[k] for k in range(Nz)], renorm if store_cumulative_result else None,
+                                    store_non_normalised_cumulative_result)
             if store_cumulative_result:
-                rn = torch.as_tensor(renorm[:Nz - 1], device=P.device)
-                self.cumulative_field = conv(rn[:, None, :] * run)  # renorm_factor(k1), :668
+                self.cumulative_field = conv(norm)
             if store_non_normalised_cumulative_result:
                 self.cumulative_field_no_norm = conv(run)
+
+
+def _cumulative(z, planes, renorm, want_running):
+    """The running z-trapezoid [Nz - 1, Nrho, No] after planes 1 .. Nz - 1 (where wanted) and, with a
+    renormalisation table, renorm_factor(k1) times it (:640-672; row k1, not k1 + 1, as in :668)."""
+    Nz, (nrho, no), dev = len(z), planes[0].shape, planes[0].device
+    step = planes[0].numel() * planes[0].element_size()
+    if not all(p.is_contiguous() and p.data_ptr() == planes[0].data_ptr() + k * step for k, p in enumerate(planes)):
+        planes = list(torch.stack(planes))  # planes of separate allocations
+    empty = lambda: torch.empty(Nz - 1, nrho, no, dtype=torch.complex128, device=dev)  # noqa: E731
+    norm, run = None if renorm is None else empty(), empty() if want_running else None
+    prob = HankelProblem(no, 2, Nz, nrho, 1.0, 0, 1, 0, 2, 0)  # only n_z, n_rho and n_omega count
+    zd = _dev(z, dev)
+    rn = None if renorm is None else _dev(renorm, dev)
+    ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+    _check(_sig().mma_hankel_cumulative(ctypes.byref(prob), zd.data_ptr(), planes[0].data_ptr(), ptr(rn), ptr(norm),
+                                        ptr(run), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)),
+           "mma_hankel_cumulative")
+    return norm, run
 
 
 def Signal_cum_integrator(ogrid, zgrid, FSourceTerm, integrator=None):
