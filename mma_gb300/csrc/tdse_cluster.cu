@@ -11,8 +11,8 @@
 //     product of them that the scan needs is computed once per instance (registers) and a scan level
 //     is one complex multiply-add;
 //   * the carry into a warp is sum_k W_k b_{g-1-k} over the earlier warps' totals with constant
-//     weights W_k = prod c, cut where |W_k| < 1e-40 (FP64) or 1e-36 (float-float): with dx = 0.1 and
-//     dt = 0.25 the solve decays by 0.77 per site and a warp of 4-site chunks needs 3 terms;
+//     weights W_k = prod c, cut where |W_k| < 1e-25: with dx = 0.1 and dt = 0.25 the solve decays by
+//     0.77 per site and a warp of 4-site chunks needs 2 terms;
 //   * each sweep is repeated from its exact carry instead of being corrected with chunk products
 //     (F, G of the CN tables): the same operation count, and no tables that depend on the chunking.
 // Warp totals travel as remote shared-memory stores to every later (forward) or earlier (backward)

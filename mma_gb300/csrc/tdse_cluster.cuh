@@ -20,18 +20,17 @@ constexpr int kMaxNC = 16;  // the largest cluster the hardware takes (over 8: o
 constexpr int kPhA = 8, kPhB = 4;  // lane = 4 a + b: e^{i F dt (4 a m dx)}, e^{i F dt (b m dx)}
 constexpr int kPh = kPhA + kPhB + kW + 1;  // + the warps' start phases + e^{-i F dt dx}
 constexpr int kPhSteps = kT / kPh;         // steps whose phases one pass of the CTA computes
+constexpr double kTiny = 1e-25;  // a warp this weakly coupled, 1e-9 of FP64's rounding, is left out of a carry
 
 // ------------------------------------------------------------------ arithmetic of the two forms
 struct Fp64 {
     typedef cd C;
     typedef double R;  // a partial sum
-    static constexpr bool kFp64 = true;
     static __device__ const C* table(const mma_tdse_grid& G) { return reinterpret_cast<const C*>(G.cn_tab); }
     static __device__ C zero() { return cd{0.0, 0.0}; }
     static __device__ C one() { return cd{1.0, 0.0}; }
     static __device__ C neg(C a) { return cd{-a.re, -a.im}; }
-    static __device__ C conj(C a) { return cd{a.re, -a.im}; }
-    static __device__ bool tiny(C a) { return fabs(a.re) + fabs(a.im) < 1e-40; }
+    static __device__ bool tiny(C a) { return fabs(a.re) + fabs(a.im) < kTiny; }
     static __device__ C mul(C a, C b) { return cmul(a, b); }
     static __device__ C fma(C a, C b, C z) { return cfma(a, b, z); }
     static __device__ C fms(C a, C b, C z) { return cfms(a, b, z); }
@@ -73,16 +72,27 @@ struct Fp64 {
     };
 };
 
+// real FP64 (the ground state): what the scans need
+struct Real64 {
+    typedef double C;
+    static __device__ C zero() { return 0.0; }
+    static __device__ C one() { return 1.0; }
+    static __device__ bool tiny(C a) { return fabs(a) < kTiny; }
+    static __device__ C mul(C a, C b) { return a * b; }
+    static __device__ C fma(C a, C b, C z) { return ::fma(a, b, z); }
+    static __device__ C shup(C v, int d) { return shfl_up(v, d); }
+    static __device__ C shdn(C v, int d) { return shfl_down(v, d); }
+    static __device__ C bcast(C v, int l) { return shfl_idx(v, l); }
+};
+
 struct Df64 {
     typedef dfk::pk C;
     typedef dfk::df R;
-    static constexpr bool kFp64 = false;
     static __device__ const C* table(const mma_tdse_grid& G) { return reinterpret_cast<const C*>(G.df_tab); }
     static __device__ C zero() { return C{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
     static __device__ C one() { return C{make_float2(1.f, 0.f), make_float2(0.f, 0.f)}; }
     static __device__ C neg(C a) { return C{dfk::ng2(a.h), dfk::ng2(a.l)}; }
-    static __device__ C conj(C a) { return C{make_float2(a.h.x, -a.h.y), make_float2(a.l.x, -a.l.y)}; }
-    static __device__ bool tiny(C a) { return fabsf(a.h.x) + fabsf(a.h.y) < 1e-36f; }
+    static __device__ bool tiny(C a) { return fabsf(a.h.x) + fabsf(a.h.y) < (float)kTiny; }
     static __device__ C mul(C a, C b) { return dfk::cmul_p(a, b); }
     static __device__ C fma(C a, C b, C z) { return dfk::cfma_p(a, b, z); }
     static __device__ C fms(C a, C b, C z) { return dfk::cfms_p(a, b, z); }

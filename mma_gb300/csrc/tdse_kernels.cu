@@ -235,8 +235,10 @@ __device__ void ground_state(const mma_tdse_grid& G, const double* tab, double* 
             double vn = (i + 1 < m) ? vq[q + kThreads] : ((t + 1 < kThreads) ? vq[t + 1] : 0.0);
             double kpsi = inv_dx2 * pc - 0.5 * inv_dx2 * (pm + pn) + (10.0 / 12.0) * pc * vc + (pm * vm + pn * vn) / 12.0;
             double mpsi = 10.0 * pc / 12.0 + (pm + pn) / 12.0;
-            acc[0] = fma(kpsi, mpsi, acc[0]);
-            acc[1] = fma(mpsi, mpsi, acc[1]);
+            if (t * m + i < n) {  // the row past the grid's end sees psi_{n-1} too, but is no row of the quotient
+                acc[0] = fma(kpsi, mpsi, acc[0]);
+                acc[1] = fma(mpsi, mpsi, acc[1]);
+            }
             pm = pc;
             pc = pn;
             vm = vc;
@@ -279,7 +281,7 @@ __device__ void ground_state(const mma_tdse_grid& G, const double* tab, double* 
 // ------------------------------------------------------------------------------------------
 // Grid builder.  mode 0: x, ground state, CN tables.  mode 1: CN tables from the grid's
 // existing x and psi0 (a caller-supplied ground state, as the legacy call1DTDSE allows).
-// mode 2 (library-internal): x and ground state only.
+// Library-internal: mode 2: x and ground state only; mode 3: x, V (in gv) and the ground state's tables.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_grid* grids, int mode)
 {
@@ -320,6 +322,7 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
         }
         chunk_products<double>(m, gtab + GS_H * L, gtab + GS_G * L, gtab + GS_F * L, gtab + GS_GG * L);
         __syncthreads();
+        if (mode == 3) return;
         // the CN table area doubles as the ground-state work space (3 L of 2*CN_SLOTS*L)
         double* work = G.cn_tab;
         ground_state(G, gtab, work, work + L, work + 2 * L, red, sc, sb, G.psi0);
@@ -565,6 +568,29 @@ using namespace mma;
 // ------------------------------------------------------------------------------------------
 // Host entry points of the batched surface.
 // ------------------------------------------------------------------------------------------
+static int sm_count()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// x and the ground states of grids with their tables: by a cluster per grid where they are few
+static bool few_ground_states(const mma_tdse_grid* grids_dev, int n_grids, int64_t max_n, cudaStream_t st)
+{
+    const int sms = sm_count();
+    if (n_grids * 4 > sms) return false;
+    build_grids_kernel<<<n_grids, kThreads, 0, st>>>(grids_dev, 3);
+    return ground_state_cluster(grids_dev, n_grids, max_n, sms, st);
+}
+
+int mma::ground_state_only(const mma_tdse_grid* grid_dev, int64_t n, cudaStream_t st)
+{
+    if (!few_ground_states(grid_dev, 1, n, st)) build_grids_kernel<<<1, kThreads, 0, st>>>(grid_dev, 2);
+    return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+}
+
 extern "C" int mma_tdse_build_grids(const mma_tdse_grid* grids_dev, const mma_tdse_grid* grids_host, int n_grids,
                                     int mode, void* stream)
 {
@@ -576,25 +602,14 @@ extern "C" int mma_tdse_build_grids(const mma_tdse_grid* grids_dev, const mma_td
             return MMA_ERR_ARG;
         if (mode == 0 && G.max_iter < 1) return MMA_ERR_ARG;
     }
+    int64_t max_n = 0;
+    for (int g = 0; g < n_grids; g++) max_n = grids_host[g].n > max_n ? grids_host[g].n : max_n;
+    if (mode == 0 && few_ground_states(grids_dev, n_grids, max_n, (cudaStream_t)stream)) mode = 1;
     build_grids_kernel<<<n_grids, kThreads, 0, (cudaStream_t)stream>>>(grids_dev, mode);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }
 
-int mma::ground_state_only(const mma_tdse_grid* grid_dev, cudaStream_t st)
-{
-    build_grids_kernel<<<1, kThreads, 0, st>>>(grid_dev, 2);
-    return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
-}
-
 static bool psi_fits_smem(int max_m) { return (size_t)max_m * kThreads * 16 <= 220 * 1024; }
-
-static int sm_count()
-{
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
 
 extern "C" int mma_tdse_propagate_c64_impl(const mma_tdse_instance* insts, int n_inst, const mma_tdse_grid* grids,
                                            const mma_tdse_buffers* bufs, int m32, int cta_threads, int grid_ctas,

@@ -48,7 +48,8 @@ def test_cluster_matches_oracle_at_chunk_edges(gpu_lib, oracle_built, num_r, dx,
 
 
 @pytest.mark.parametrize("precision, tol", [("fp64", 1e-10), ("df64", 1e-9)])
-@pytest.mark.parametrize("num_r, n_inst", [(601, 2), (1203, 5), (8000, 9), (8000, 41), (30000, 2)])
+@pytest.mark.parametrize("num_r, n_inst", [(601, 2), (1203, 5), (6000, 2), (10000, 2), (12500, 3), (8000, 9), (8000, 41),
+                                            (30000, 2)])
 def test_cluster_matches_one_cta_kernel(gpu_lib, precision, tol, num_r, n_inst):
     from mma_gb300.tdse_batch import TDSEGrids, run_batch
 
@@ -126,7 +127,8 @@ class _OneCta:
 
 
 @pytest.mark.parametrize("num_r, dx, K", [(4, 0.4, 8), (127, 0.3, 7), (128, 0.3, 1), (640, 0.2, 64), (2047, 0.2, 9),
-                                          (8000, 0.1, 32), (1500, 0.02, 16)])
+                                          (8000, 0.1, 32), (1500, 0.02, 16), (3000, 0.1, 20), (6000, 0.1, 16),
+                                          (10000, 0.1, 16), (13000, 0.1, 16)])
 def test_adjoint_cluster_matches_one_cta_kernel(gpu_lib, monkeypatch, num_r, dx, K):
     """The cluster form of the adjoint sweep (segments that end inside a batch of phases or of collected
     sums, chunks of one site, threads without sites): 1e-10, as for the propagation."""
@@ -145,3 +147,31 @@ def test_adjoint_cluster_matches_one_cta_kernel(gpu_lib, monkeypatch, num_r, dx,
     assert rel_l2(L.cpu().numpy(), L1.cpu().numpy()) < 1e-10
     for i in range(2):
         assert rel_l2(g[i].cpu().numpy(), g1[i].cpu().numpy()) < 1e-10, i
+
+
+@pytest.mark.parametrize("num_r, dx", [(2, 0.4), (40, 0.4), (127, 0.3), (128, 0.3), (513, 0.3), (2048, 0.2), (8000, 0.1),
+                                       (12001, 0.1), (33000, 0.05), (6000, 0.1), (4100, 0.1), (10000, 0.1), (14000, 0.1)])
+def test_ground_state_cluster(gpu_lib, oracle_built, num_r, dx):
+    """One grid (a cluster) against the oracle and against the same grid among 40 (a CTA per grid).  The
+    iterations stop on |dE| <= 1e-15: on small grids two orders of summation leave the energies 1e-11
+    apart (tests/test_edges_gpu.py), and one iteration more or less changes psi0 by 1e-11."""
+    import oracle.tdse as ot
+    from mma_gb300.tdse_batch import TDSEGrids
+
+    p = dict(num_r=num_r, dx=dx, trg_a=A_CONFIG)
+    one = TDSEGrids([p], dt=0.25)
+    x, psi0, e, _ = ot.ground_state(num_r, dx, A_CONFIG, -1.0, 1e-15)
+    assert abs(one.Einit[0] - e) < 1e-10 * abs(e)
+    assert rel_l2(one.psi0(0).cpu().numpy(), psi0) < 1e-9
+    assert np.array_equal(one.x(0).cpu().numpy(), x)
+    if num_r <= 2048:
+        many = TDSEGrids([p] * 40, dt=0.25)
+        assert abs(one.Einit[0] - many.Einit[17]) < 1e-10 * abs(e)
+        assert rel_l2(one.psi0(0).cpu().numpy(), many.psi0(17).cpu().numpy()) < 1e-9
+
+
+def test_ground_state_cluster_iteration_cap(gpu_lib):
+    from mma_gb300.tdse_batch import MMAStatusError, TDSEGrids
+
+    with pytest.raises(MMAStatusError, match="not converged"):
+        TDSEGrids([dict(num_r=600, dx=0.4, trg_a=A_CONFIG, max_iter=3)], dt=0.25)
