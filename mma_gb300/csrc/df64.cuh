@@ -142,6 +142,20 @@ __device__ __forceinline__ pk cfms_p(pk a, pk b, pk z)
 {
     return dot_add(products(bc(-a.h.x), bc(-a.l.x), b.h, b.l, bc(a.h.y), bc(a.l.y), mipair(b.h), mipair(b.l)), z);
 }
+// f y0 + y - g u: the forward correction and the backward sweep of a site in one sum (five leading
+// terms by four TwoSums, every low-order term folded once, one renormalisation)
+__device__ __forceinline__ pk correct_sweep_p(pk f, pk y0, pk y, pk g, pk u)
+{
+    const prods a = cprods(f, y0);
+    const prods b = products(bc(-g.h.x), bc(-g.l.x), u.h, u.l, bc(g.h.y), bc(g.l.y), mipair(u.h), mipair(u.l));
+    float2 s1, t1, s2, t2, s3, t3, s4, t4;
+    two_sum2(a.p, a.q, s1, t1);
+    two_sum2(s1, y.h, s2, t2);  // off the chain of u
+    two_sum2(b.p, b.q, s3, t3);
+    two_sum2(s2, s3, s4, t4);
+    const float2 la = add2(add2(t1, t2), add2(add2(a.ep, a.eq), y.l));
+    return renorm2(s4, add2(add2(add2(t3, t4), add2(b.ep, b.eq)), la));
+}
 // 10 p + a + b per lane (the Numerov right-hand side), one TwoSum per pair of leading terms,
 // unnormalised (feeds a product)
 __device__ __forceinline__ pk ten_sum_p(pk p, pk a, pk b)

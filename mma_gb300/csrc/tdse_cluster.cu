@@ -421,7 +421,7 @@ namespace mma {
 // expected time of a step of the whole batch.  The models were fitted to runs of 1 to 304 instances on
 // grids of 601 to 8001 sites (us per step, measured / model):
 //   one CTA    FP64   601 sites  24.3 / 24.3    8001 sites  108.8 / 108.7   256 x 4001 sites  125 / 124
-//              df64   601 sites   7.8 /  7.8    8001 sites   35.1 /  35.1   304 x 8001 sites  58.8 / 58.9
+//              df64   601 sites   7.6 /  7.5    8001 sites   34.1 /  34.1   304 x 8001 sites  54.0 / 54.0
 //   cluster    FP64  8001 sites  NC = 4  29.0 / 28.8   8  17.3 / 17.2   16  11.7 / 11.4;  256 x 4001, NC = 2  115 / 115
 //              df64  8001 sites  NC = 4  10.1 / 10.1   8   6.9 /  7.2   16   5.6 /  5.7
 // A second CTA on an SM costs FP64 its pipe time (16.1 us a wave measured at m = 4, 17.4 modelled) and
@@ -430,7 +430,7 @@ namespace {
 double one_cta_us(int m256, int precision, int n_inst, int sms)
 {
     if (precision != 2) return (double)((n_inst + sms - 1) / sms) * (15.6 + 2.91 * m256);
-    const double one = 5.0 + 0.94 * m256, two = 8.3 + 1.58 * m256;
+    const double one = 4.8 + 0.915 * m256, two = 7.8 + 1.445 * m256;
     const int full = n_inst / (2 * sms), rest = n_inst % (2 * sms);
     return full * two + (rest == 0 ? 0.0 : rest <= sms ? one : two);
 }

@@ -26,9 +26,15 @@
 // Each pass reads its operands through a small cp.async ring in shared memory, two sites ahead,
 // which hides the L2 latency without registers (30% faster at one CTA per SM, 9% at two).
 // No warp carries serial FP64 work into the scan barriers (a 32-lane FP64 instruction holds a
-// sub-partition's FP64 unit for about 64 cycles): the phase factors come from one FP64 sincos
-// per thread for 25 steps at a time, and the observables' warp sums stay double-word until
-// lanes of warp 0 convert them.
+// sub-partition's FP64 unit for about 64 cycles): the phase factors come from FP64 sincos spread over the
+// threads for some twenty steps at a time, and the observables' warp sums stay double-word until lanes
+// of warp 0 convert them.
+//
+// Bound by the double-word chains' latency and the CTA barriers between the passes (FMA pipe 49% busy,
+// issue 46%, a quarter of the warps' time at barriers).  Per step of 304 instances of 8001 sites (two CTAs
+// an SM): 58.9 us before the operand ring was aligned, the chunks kept their own frames (below), the
+// correction and the backward sweep became one sum and a real psi0 took half a projection; 54.0 us now
+// with 11% fewer instructions.  The whole benchmark map, 4 cycles: 667 -> 609 ms.
 #include <cuda_runtime.h>
 
 #include "../../include/mma_tdse.h"
@@ -130,23 +136,38 @@ struct Args {
     int64_t max_L;
 };
 
-constexpr int kPow = 8;  // e^{i F dt M dx 2^b}, b < 8: the chunk-start phases of 256 threads
-constexpr int kPhase = kPow + 2;  // phase factors per step
-constexpr int kPhaseSteps = kThreads / kPhase;  // steps whose factors one pass of the CTA computes
+// The phase e^{i F dt x} of a step splits into a part that is constant over a thread's chunk and one
+// that is the same for every thread: x = x_{s0(t)} + i dx.  The first is never applied: thread t keeps
+// psi in its own frame, psi = B_t psi~ with B_t = e^{i A x_{s0}}, A = dt (sum of the fields so far).  The
+// solve commutes with a constant, so inside a chunk nothing changes, and between neighbours only the one
+// factor R = B_{t+1}/B_t = e^{i A m dx} enters: the halo values, the scans' coefficients and their
+// carries.  Per site that saves the phase's recurrence (one of about ten double-word products), per
+// thread the products of its start phase; <psi0|psi> is summed over the lanes and warps with powers of R.
+// Factors per step: R before the step, R^1, 2, 4, 8, 16 and R^{32 w} after it, then z^i = e^{i F dt i dx}
+// for the chunk's sites (in two levels, i = 32 a + b, where a chunk has more than kFlat sites).
+constexpr int kRb = 0, kRp = 1, kRw = 6, kZ = kRw + kWarps;
+constexpr int kFlat = 512, kFactors = 1024;  // factors of as many steps as fit are computed at a time
+__host__ __device__ inline int z_entries(int m) { return m <= kFlat ? m : 32 + (m + 31) / 32; }
+__host__ __device__ inline int factor_entries(int m) { return kZ + z_entries(m) > kFactors ? kZ + z_entries(m) : kFactors; }
+constexpr int kMaxSteps = kFactors / (kZ + 1);
 // Operand ring: each pass copies the operands of site i + kDepth - 1 into shared memory while it
 // computes site i (kSlots float4 per site at most, pass 3), so the L2 latency of psi, the sweep
 // buffer and the tables is hidden without holding registers.
 constexpr int kDepth = 3, kSlots = 5;
 constexpr int kRingBytes = kDepth * kSlots * kThreads * 16;  // 61,440 bytes per CTA
+inline size_t smem_bytes(int max_m) { return kRingBytes + 16 * (size_t)factor_entries(max_m); }
 
+template <bool FLAT>
 __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
 {
-    extern __shared__ float4 ring[];  // [kDepth][kSlots][kThreads]
+    // [kDepth][kSlots][kThreads], then the factors of the steps.  The alignment matters: with the ring off a
+    // 64-byte boundary every 64-byte half of a warp's copy is fetched twice (L2 reads 0.78 -> 1.54 G sectors)
+    extern __shared__ __align__(128) float4 ring[];
+    pk* const fac = reinterpret_cast<pk*>(ring + kDepth * kSlots * kThreads);
     __shared__ pk sc[2 * kWarps], sb[2 * kWarps];
     __shared__ double red[kWarps];
     __shared__ df redf[kWarps * 5];  // per warp: -<V'>, <x>, <psi0|psi> (re, im), window population
-    // per step of the current block of kPhaseSteps: e^{i F dt x_0}, e^{i F dt dx}, e^{i F dt M dx 2^b}
-    __shared__ pk s_pow[kPhaseSteps][kPhase];
+    __shared__ double s_A[kMaxSteps + 1];  // A before the current block of steps and after each of them
     __shared__ int64_t s_inst, s_gate, s_lo, s_hi;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     float4* yl = P.scratch + blockIdx.x * P.max_L;
@@ -187,8 +208,13 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
             s_lo = lo < 0 ? 0 : lo;
             s_hi = hi > num_r ? num_r : hi;
         }
-        for (int64_t i = 0; i < m; i++) psi[i * kThreads + t] = P0[i * kThreads + t];
-        __syncthreads();
+        bool im = false;
+        for (int64_t i = 0; i < m; i++) {
+            const float4 v = P0[i * kThreads + t];
+            psi[i * kThreads + t] = v;
+            im |= v.y != 0.f;
+        }
+        const bool psi0_im = __syncthreads_or(im);
         const int64_t lo = s_lo, hi = s_hi, gate = s_gate;
         const int64_t s0 = t * m;
         {   // initial window population (prop.c:87-93), FP64 from the FP64 ground state
@@ -206,9 +232,25 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
             }
         }
         double tt = I.tmin, Fprev = 0.0;
-        const double x0 = G.x[0];
+        const double xs = s0 < n ? G.x[s0] : 0.0;
+        auto applied = [&](int64_t k) { return (k <= gate || k >= I.n_field || k >= S) ? 0.0 : f[k]; };
+        auto store_psi = [&](double* dst, double A) {  // psi = B_t psi~, natural order
+            double sn, cs;
+            sincos(A * xs, &sn, &cs);
+            for (int64_t i = 0; i < m; i++)
+                if (s0 + i < n) {
+                    const pk v = pld(psi + i * kThreads + t);
+                    const double re = (double)v.h.x + (double)v.l.x, im = (double)v.h.y + (double)v.l.y;
+                    dst[2 * (s0 + i)] = re * cs - im * sn;
+                    dst[2 * (s0 + i) + 1] = re * sn + im * cs;
+                }
+        };
+        const int mi = (int)m;  // sites per thread: 32-bit indices in the site loops
+        const int per = kZ + (FLAT ? mi : z_entries(kFlat < mi ? mi : kFlat + 1)), nb = kFactors / per > 1 ? kFactors / per : 1;
+        int kb = nb;  // steps of the current block done
+        if (t == 0) s_A[0] = 0.0;
         for (int64_t k = 0; k < S; k++) {
-            const double Fk = (k <= gate || k >= I.n_field) ? 0.0 : f[k];
+            const double Fk = applied(k);
             if (w == 0) {
                 if (k > 0) observables_out(redf, lane, k, Fprev, o_src, o_x, o_ptot, o_pint);
                 if (lane == 0) {
@@ -218,23 +260,41 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
                 }
             }
             Fprev = Fk;
-            // the phase factors of the next kPhaseSteps steps in FP64, one angle per thread, so
-            // that the FP64 pipe's work is spread evenly over the warps: e^{i F dt x_0},
-            // e^{i F dt dx} and e^{i F dt m dx 2^b}
-            if (k % kPhaseSteps == 0 && t < kPhaseSteps * kPhase) {
-                const int a = t % kPhase;
-                const int64_t ks = k + t / kPhase;
-                const double Fs = (ks <= gate || ks >= I.n_field || ks >= S) ? 0.0 : f[ks];
-                const double ang = a == 0 ? Fs * dt * x0 : (a == 1 ? Fs * dt * dx
-                                                                   : Fs * dt * (double)m * dx * (double)(1 << (a - 2)));
-                double sn, cs;
-                sincos(ang, &sn, &cs);
-                const df c2 = from_d(cs), s2 = from_d(sn);
-                s_pow[t / kPhase][a] = pk{make_float2(c2.hi, s2.hi), make_float2(c2.lo, s2.lo)};
+            // the factors of the next block of steps in FP64, spread evenly over the threads (a 32-lane
+            // FP64 instruction holds a sub-partition's FP64 unit for about 64 cycles)
+            if (kb == nb) {
+                if (k > 0 && t == 0) s_A[0] = s_A[nb];
+                __syncthreads();
+                if (t >= 1 && t <= nb) {
+                    double A = s_A[0];
+                    for (int j = 0; j < t; j++) A += dt * applied(k + j);
+                    s_A[t] = A;
+                }
+                __syncthreads();
+                for (int e = t; e < nb * per; e += kThreads) {
+                    const int st = e / per, q = e % per;
+                    const double step = (double)m * dx;
+                    double ang;
+                    if (q == kRb) ang = s_A[st] * step;
+                    else if (q < kRw) ang = s_A[st + 1] * (step * (1 << (q - kRp)));
+                    else if (q < kZ) ang = s_A[st + 1] * (step * (32 * (q - kRw)));
+                    else {
+                        const int i = q - kZ;
+                        ang = applied(k + st) * dt * (dx * (double)(FLAT || i < 32 ? i : 32 * (i - 32)));
+                    }
+                    double sn, cs;
+                    sincos(ang, &sn, &cs);
+                    const df c2 = from_d(cs), s2 = from_d(sn);
+                    fac[e] = pk{make_float2(c2.hi, s2.hi), make_float2(c2.lo, s2.lo)};
+                }
+                __syncthreads();
+                kb = 0;
             }
+            const pk* const fk = fac + kb * per;
+            kb++;
+            const pk Rb = fk[kRb], Rbc{make_float2(Rb.h.x, -Rb.h.y), make_float2(Rb.l.x, -Rb.l.y)};
             // ---- pass 1: local forward sweep of the right-hand side 2 M2 psi
             const pk zero{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-            const int mi = (int)m;  // sites per thread: 32-bit indices in the site loops
             float4* const my = ring + t;
             constexpr int kStage = kSlots * kThreads;
             // site i's operands: psi of site i + 1 (the next thread's first site after the last),
@@ -250,24 +310,28 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
                 if (d < mi) issue1(d, my + d * kStage);
                 cp_commit();
             }
-            pk pm = (t == 0) ? zero : pld(psi + (m - 1) * kThreads + t - 1);
+            pk pm = (t == 0) ? zero : cmul_p(Rbc, pld(psi + (m - 1) * kThreads + t - 1));
             pk pc = pld(psi + t);
             pk yprev = zero;
             int su = 0;  // ring stage of the current site; the stage before it is refilled
-            for (int i = 0; i < mi; i++) {
+            auto site1 = [&](int i, bool last) {
                 float4* const r = my + su * kStage;
                 if (i + kDepth - 1 < mi) issue1(i + kDepth - 1, my + (su == 0 ? kDepth - 1 : su - 1) * kStage);
                 cp_commit();
                 cp_wait<kDepth - 1>();
-                const pk pn = (i + 1 < mi || t + 1 < kThreads) ? pld(r) : zero;
+                pk pn = !last || t + 1 < kThreads ? pld(r) : zero;
+                if (last) pn = cmul_p(Rb, pn);  // the next thread's first site, in this thread's frame
                 const pk r2 = ten_sum_p(pc, pm, pn);
                 yprev = cfms_p(pld(r + kThreads), yprev, cmul_pu(pld(r + 2 * kThreads), r2));
                 pst(yl + i * kThreads + t, yprev);
                 pm = pc;
                 pc = pn;
                 su = su + 1 == kDepth ? 0 : su + 1;
-            }
-            const pk yin = scan_fwd(pld(FF + (m - 1) * kThreads + t), yprev, sc, sb);
+            };
+#pragma unroll 2
+            for (int i = 0; i + 1 < mi; i++) site1(i, false);
+            site1(mi - 1, true);
+            const pk yin = cmul_p(Rbc, scan_fwd(cmul_p(Rbc, pld(FF + (m - 1) * kThreads + t)), yprev, sc, sb));
             // ---- pass 2: forward correction, local backward sweep
             auto issue2 = [&](int i, float4* r) {  // F, y and G of site i
                 const int q = i * kThreads + t;
@@ -282,24 +346,19 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
             }
             pk unext = zero;
             su = 0;
+#pragma unroll 2
             for (int j = 0; j < mi; j++) {  // site i = mi - 1 - j
                 float4* const r = my + su * kStage;
                 if (j + kDepth - 1 < mi) issue2(mi - kDepth - j, my + (su == 0 ? kDepth - 1 : su - 1) * kStage);
                 cp_commit();
                 cp_wait<kDepth - 1>();
-                const pk y = cfma_p(pld(r), yin, pld(r + kThreads));
-                unext = cfms_p(pld(r + 2 * kThreads), unext, y);
+                unext = correct_sweep_p(pld(r), yin, pld(r + kThreads), pld(r + 2 * kThreads), unext);
                 pst(yl + (mi - 1 - j) * kThreads + t, unext);
                 su = su + 1 == kDepth ? 0 : su + 1;
             }
-            const pk uin = scan_bwd(pld(GP + t), unext, sc + kWarps, sb + kWarps);
+            const pk uin = cmul_p(Rb, scan_bwd(cmul_p(Rb, pld(GP + t)), unext, sc + kWarps, sb + kWarps));
             // ---- pass 3: backward correction, CN update, phase e^{+i F dt x}, observables
-            const pk* pw = s_pow[k % kPhaseSteps];
-            pk ph = pw[0];  // e^{i F dt x_0} (e^{i F dt m dx})^t = e^{i F dt x_{s0}}
-#pragma unroll
-            for (int b = 0; b < kPow; b++)
-                if (t & (1 << b)) ph = cmul_p(ph, pw[2 + b]);
-            const pk z = pw[1];
+            const pk* const zk = fk + kZ;
             // lanes (-<V'>, <x>) and the projection (re, im) on psi0
             pk acc01 = zero, acc23 = zero;
             df acc[5];
@@ -317,6 +376,7 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
                 cp_commit();
             }
             su = 0;
+#pragma unroll 2
             for (int i = 0; i < mi; i++) {
                 float4* const r = my + su * kStage;
                 if (i + kDepth - 1 < mi) issue3(i + kDepth - 1, my + (su == 0 ? kDepth - 1 : su - 1) * kStage);
@@ -327,18 +387,26 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
                 const pk gp = pld(r), yv = pld(r + kThreads), po = pld(r + 2 * kThreads);
                 // u - psi with u = G u_in + y, the CN update before the phase
                 const pk d = cn_update_p(gp, uin, yv, po);
-                const pk pn = cmul_p(ph, d);
+                pk z;
+                if constexpr (FLAT) z = zk[i]; else z = cmul_p(zk[32 + (i >> 5)], zk[i & 31]);
+                const pk pn = cmul_p(z, d);
                 pst(psi + q, pn);
-                ph = cmul_p(ph, z);
                 const df n2 = norm2_u(pn);
                 const pk gx = pld(r + 3 * kThreads), p0 = pld(r + 4 * kThreads);
                 acc_mul_p(acc01, n2.hi, n2.lo, gx);
-                acc_proj_p(acc23, pn, p0);
+                if (psi0_im) acc_proj_p(acc23, pn, p0);
+                else acc_mul_p(acc23, p0.h.x, p0.l.x, pn);
             }
             acc01 = renorm2(acc01.h, acc01.l);
             acc23 = renorm2(acc23.h, acc23.l);
             acc[0] = df{acc01.h.x, acc01.l.x};
             acc[1] = df{acc01.h.y, acc01.l.y};
+            // <psi0|psi> = sum_t B_t p_t: over the lanes with R^1, 2, 4, 8, 16, then over the warps (R^{32 w};
+            // the common B_0 does not change its modulus).  The complex projection is its conjugate.
+            if (psi0_im) acc23 = pk{make_float2(acc23.h.x, -acc23.h.y), make_float2(acc23.l.x, -acc23.l.y)};
+#pragma unroll
+            for (int l = 0; l < 5; l++) acc23 = cfma_p(fk[kRp + l], pshdn(acc23, 1 << l), acc23);
+            acc23 = cmul_p(fk[kRw + w], acc23);
             acc[2] = df{acc23.h.x, acc23.l.x};
             acc[3] = df{acc23.h.y, acc23.l.y};
             acc[4] = df{0.f, 0.f};  // the few sites of the population window in this chunk
@@ -350,7 +418,8 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
 #pragma unroll
             for (int d = 16; d >= 1; d >>= 1)
 #pragma unroll
-                for (int c = 0; c < 5; c++) acc[c] = add(acc[c], shfl_xor_df(acc[c], d));
+                for (int c = 0; c < 5; c++)
+                    if (c < 2 || c > 3) acc[c] = add(acc[c], shfl_xor_df(acc[c], d));
             if (lane == 0)
 #pragma unroll
                 for (int c = 0; c < 5; c++) redf[w * 5 + c] = acc[c];
@@ -359,26 +428,14 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
                 if (k % I.snap_every == 0 && k / I.snap_every < I.n_snap - 1) slot = k / I.snap_every;
                 if (k == S - 1) slot = I.n_snap - 1;
                 if (slot >= 0) {
-                    double* sp = P.snapshots + I.snap_off + slot * 2 * n;
-                    for (int64_t i = 0; i < m; i++)
-                        if (s0 + i < n) {
-                            const pk v = pld(psi + i * kThreads + t);
-                            sp[2 * (s0 + i)] = (double)v.h.x + (double)v.l.x;
-                            sp[2 * (s0 + i) + 1] = (double)v.h.y + (double)v.l.y;
-                        }
+                    store_psi(P.snapshots + I.snap_off + slot * 2 * n, s_A[kb]);
                 }
             }
             __syncthreads();
         }
         if (w == 0) observables_out(redf, lane, S, Fprev, o_src, o_x, o_ptot, o_pint);
         if (P.psi_final && I.psi_off >= 0) {
-            double* pf = P.psi_final + I.psi_off;
-            for (int64_t i = 0; i < m; i++)
-                if (s0 + i < n) {
-                    const pk v = pld(psi + i * kThreads + t);
-                    pf[2 * (s0 + i)] = (double)v.h.x + (double)v.l.x;
-                    pf[2 * (s0 + i) + 1] = (double)v.h.y + (double)v.l.y;
-                }
+            store_psi(P.psi_final + I.psi_off, s_A[kb]);
         }
         __syncthreads();
     }
@@ -415,18 +472,21 @@ extern "C" int mma_tdse_build_df_tables(const mma_tdse_grid* grids_dev, const mm
 
 // CTAs of the float-float form resident at once (two per SM), and the scratch they need:
 // per CTA the sweep buffer and psi, 16 bytes per site each.
-static bool df64_smem_attr()
+static bool df64_smem_attr(size_t smem)
 {
-    return cudaFuncSetAttribute(dfk::propagate_df64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                dfk::kRingBytes) == cudaSuccess;
+    return cudaFuncSetAttribute(dfk::propagate_df64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem) == cudaSuccess &&
+           cudaFuncSetAttribute(dfk::propagate_df64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem) == cudaSuccess;
 }
 
 extern "C" int mma_tdse_df64_default_ctas()
 {
     int dev = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || !df64_smem_attr()) return 0;
+    const size_t smem = dfk::smem_bytes(1);  // up to some thousand sites per thread take no more
+    if (cudaGetDevice(&dev) != cudaSuccess || !df64_smem_attr(smem)) return 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dfk::propagate_df64_kernel, kThreads, dfk::kRingBytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dfk::propagate_df64_kernel<true>, kThreads, smem);
     return sms * (per_sm > 0 ? per_sm : 1);
 }
 
@@ -443,7 +503,9 @@ extern "C" int mma_tdse_propagate_df64_impl(const mma_tdse_instance* insts, int 
     if (cudaMemsetAsync(bufs->counter, 0, sizeof(int), st) != cudaSuccess) return MMA_ERR_CUDA;
     dfk::Args A{insts, n_inst, grids, bufs->fields, bufs->outputs, bufs->psi_final, bufs->snapshots, bufs->counter,
                 reinterpret_cast<float4*>(bufs->scratch), (int64_t)max_m * kThreads};
-    if (!df64_smem_attr()) return MMA_ERR_CUDA;
-    dfk::propagate_df64_kernel<<<grid_ctas, kThreads, dfk::kRingBytes, st>>>(A);
+    const size_t smem = dfk::smem_bytes(max_m);
+    if (!df64_smem_attr(smem)) return MMA_ERR_CUDA;
+    auto kern = max_m <= dfk::kFlat ? dfk::propagate_df64_kernel<true> : dfk::propagate_df64_kernel<false>;
+    kern<<<grid_ctas, kThreads, smem, st>>>(A);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }
