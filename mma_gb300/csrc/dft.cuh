@@ -29,6 +29,11 @@ int get_plan(int n, cudaStream_t st, const Plan** out);
 int r2c(const Plan* p, const double* x, int64_t x_stride, double2* X, int64_t X_stride, int n_batch,
         cudaStream_t st);
 
+// norm |r2c(win_w sig_s)_k| for k < nf into g[s n_win + w][nf] (signals at sig + s stride, windows [n_win][n],
+// nf <= n/2 + 1) where rows fit in shared memory; false, and nothing launched, where they do not.
+bool windowed(const Plan* p, const double* sig, int64_t stride, int n_sig, const double* win, int n_win, int nf,
+              double norm, double* g, cudaStream_t st);
+
 // c2r of n_batch rows from the first n_bins bins of each X row (bins n_bins .. n/2 are zero),
 // times `scale`.  The global-memory path (FFT length above 7168) takes its two work buffers
 // from the stream-ordered allocator.

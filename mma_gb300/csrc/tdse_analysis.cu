@@ -484,11 +484,15 @@ extern "C" int mma_gabor(const double* signals, int64_t stride, int n_sig, doubl
     // the window table sits at the front of the DFT output buffer: it is read before the DFT writes there
     double* win = reinterpret_cast<double*>(out);
     an::gabor_table<<<an::grid_for((int64_t)N_G * N), 256, 0, st>>>(N, N_G, dt, t_min, dt_G, ia, win);
-    an::gabor_window<<<an::grid_for(nb * N), 256, 0, st>>>(signals, stride, n_sig, N, N_G, win, in);
     const mma::dft::Plan* p = nullptr;
     int rc = mma::dft::get_plan(N, st, &p);
-    if (rc == MMA_OK) rc = mma::dft::r2c(p, in, N, out, Nc, (int)nb, st);
     if (rc != MMA_OK) return rc;
-    an::gabor_abs<<<an::grid_for(nb * N_freq), 256, 0, st>>>(out, Nc, nb, N_freq, dt / sqrt(2. * an::kPi), gabor);
+    const double norm = dt / sqrt(2. * an::kPi);
+    if (mma::dft::windowed(p, signals, stride, n_sig, win, N_G, N_freq, norm, gabor, st))
+        return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+    an::gabor_window<<<an::grid_for(nb * N), 256, 0, st>>>(signals, stride, n_sig, N, N_G, win, in);
+    rc = mma::dft::r2c(p, in, N, out, Nc, (int)nb, st);
+    if (rc != MMA_OK) return rc;
+    an::gabor_abs<<<an::grid_for(nb * N_freq), 256, 0, st>>>(out, Nc, nb, N_freq, norm, gabor);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }
