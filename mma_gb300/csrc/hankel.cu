@@ -968,7 +968,7 @@ int launch_fast(const mma_hankel_problem* p, const mma_hankel_fast_plan_t* plan,
     const size_t consts = (ser ? MM * (sizeof(float2) + 2 * sizeof(float4)) : MM * sizeof(float4));
     int rtile = (int)(p->n_r < 512 ? p->n_r : 512);
     rtile += rtile & 1;  // even row stride: stage 2 loads radius pairs as 16-byte words
-    while ((size_t)rows * rtile * sizeof(float2) + consts > budget && rtile > 32) rtile /= 2;
+    while ((size_t)rows * rtile * sizeof(float2) + consts > budget && rtile > 32) rtile = (rtile / 2 + 1) & ~1;
     const size_t s2 = (size_t)rows * rtile * sizeof(float2) + consts;
     dim3 g2((unsigned)((p->n_rho + kThreads - 1) / kThreads), (unsigned)p->n_omega);
     const float cut8 = series_cut(plan, MM - 8), cut4 = series_cut(plan, MM - 4);
