@@ -421,12 +421,27 @@ __global__ void __launch_bounds__(kThreads) fast_stage1(mma_hankel_problem P, co
 // series), with A_k from series_plane_a and the pairs (v_k0^m, v_k1^m) from series_plane_tables;
 // the planes' sums run as FP32x2 pairs (one lane per plane) beside the far field's.
 constexpr int kSeriesPlanes = 2;
+// What bounds it: the FP32 pipe (packed instructions hold it two cycles; it is 67% active, the issue
+// slots 61%).  Two radius pairs per step share each coefficient, which a packed instruction wants
+// as a register pair, and run as two interleaved chains; the series lengths share one unrolled chain of terms, left early
+// where a chunk needs fewer (three copies of it overflowed the instruction cache: one pair per step
+// and a copy per length 1.55 ms, two pairs with copies 1.75 ms, two pairs and one chain 1.49 ms).
+// Blocks of 128, four per SM: n_rho <= 128 leaves no idle half, and the blocks stage their tiles at
+// different times.  2048 frequencies, 512 radii, 256 rho, two planes: 1.76 -> 1.49 ms.
+constexpr int kS2Threads = 128, kS2Pairs = 2;
+// the recurrence's constants per term as broadcast pairs, (s m/(m+1), the same, -1/(m(m+1)), the same):
+// a kernel argument, read from the constant bank
+template <int MM>
+struct stage2_terms {
+    float4 c[MM];
+};
 template <int MM, bool SER>
-__global__ void __launch_bounds__(kThreads, SER ? 2 : 3) fast_stage2(mma_hankel_problem P, mma_hankel_fast_plan_t F,
+__global__ void __launch_bounds__(kS2Threads, 4) fast_stage2(mma_hankel_problem P, mma_hankel_fast_plan_t F,
                                                         const double* og, const double* rg, const double* rho,
                                                         const float2* Bp, double2* ff, int rtile,
                                                         const float2* asel, const float2* vsel, int n_sel,
-                                                        double2* planes, float x_cut8, float x_cut4)
+                                                        double2* planes, float x_cut8, float x_cut4,
+                                                        const __grid_constant__ stage2_terms<MM> T)
 {
     extern __shared__ __align__(16) float smem[];
     const int64_t o = blockIdx.y, Nr = P.n_r, Nrho = P.n_rho, No = P.n_omega;
@@ -435,17 +450,12 @@ __global__ void __launch_bounds__(kThreads, SER ? 2 : 3) fast_stage2(mma_hankel_
     float2* kr = reinterpret_cast<float2*>(B4 + MM * (rtile / 2));  // rtile
     float2* As = kr + rtile;                       // SER: kSeriesPlanes * rtile, A_k of the selected planes
     float2* Vs = As + kSeriesPlanes * rtile;       // SER: MM pairs (v_k0^m, v_k1^m)
-    // per term m the recurrence's constants as broadcast pairs (s m/(m+1), -1/(m(m+1))) and, with
-    // SER, the planes' (v_k0^m, v_k1^m) as broadcast pairs: read whole by one 16-byte load
-    float4* Cm = reinterpret_cast<float4*>(kr + rtile + (SER ? kSeriesPlanes * rtile + MM : 0));
-    float4* Vb = Cm + MM;  // SER
-    const uint32_t cm_s = (uint32_t)__cvta_generic_to_shared(Cm), vb_s = cm_s + 16u * MM;
+    // with SER the planes' (v_k0^m, v_k1^m) per term as broadcast pairs, read whole by one 16-byte load
+    float4* Vb = reinterpret_cast<float4*>(kr + rtile + (SER ? kSeriesPlanes * rtile + MM : 0));
+    const uint32_t vb_s = (uint32_t)__cvta_generic_to_shared(Vb);
     const float s = (float)F.sigma;
-    for (int m = threadIdx.x; m < MM; m += blockDim.x) {
-        const float c1 = s * __fdiv_rn((float)m, (float)(m + 1));
-        const float c2 = m > 0 ? -__fdiv_rn(1.0f, (float)(m * (m + 1))) : 0.f;
-        Cm[m] = make_float4(c1, c1, c2, c2);
-        if (SER) {
+    if (SER) {
+        for (int m = threadIdx.x; m < MM; m += kS2Threads) {
             const float2 v = vsel[m];
             Vs[m] = v;
             Vb[m] = make_float4(v.x, v.x, v.y, v.y);
@@ -455,7 +465,7 @@ __global__ void __launch_bounds__(kThreads, SER ? 2 : 3) fast_stage2(mma_hankel_
 #pragma unroll
     for (int i = 0; i < kSeriesPlanes; i++) ppart[i] = phi[i] = plo[i] = make_float2(0.f, 0.f);
     const double kap = (og[o] / kC) / F.d_ref;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t j = blockIdx.x * (int64_t)kS2Threads + threadIdx.x;
     float rh = 0.f, rl = 0.f;
     if (j < Nrho) split_d(rho[j], rh, rl);
     // the series length per (warp, chunk of kChunk radii): sigma y / 2 <= x_cut8 (x_cut4) lets MM - 8
@@ -469,14 +479,22 @@ __global__ void __launch_bounds__(kThreads, SER ? 2 : 3) fast_stage2(mma_hankel_
     for (int64_t r0 = 0; r0 < Nr; r0 += rtile) {
         const int64_t nt = (Nr - r0 < rtile) ? (Nr - r0) : rtile;
         __syncthreads();
-        for (int64_t q = threadIdx.x; q < MM * nt; q += blockDim.x) {
-            const int64_t m = q / nt, rr = q % nt;
-            const float2 v = Bp[(o * MM + m) * Nr + r0 + rr];
-            float* w = reinterpret_cast<float*>(B4 + m * (rtile / 2) + rr / 2) + (rr & 1);
-            w[0] = v.x;
-            w[2] = v.y;
+        const int np = (int)(nt + 1) / 2, warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+        for (int m = warp; m < MM; m += kS2Threads / 32) {
+            const float2* const b = Bp + (o * MM + m) * Nr + r0;
+#pragma unroll 4
+            for (int p = lane; p < np; p += 32) {
+                float4 v;
+                if (!(Nr & 1)) {
+                    v = reinterpret_cast<const float4*>(b)[p];  // r0 is even, Bp 256-byte aligned
+                } else {
+                    const float2 v0 = b[2 * p], v1 = 2 * p + 1 < nt ? b[2 * p + 1] : make_float2(0.f, 0.f);
+                    v = make_float4(v0.x, v0.y, v1.x, v1.y);
+                }
+                B4[m * (rtile / 2) + p] = make_float4(v.x, v.z, v.y, v.w);
+            }
         }
-        for (int64_t q = threadIdx.x; q < nt; q += blockDim.x) {
+        for (int q = threadIdx.x; q < nt; q += kS2Threads) {
             float h, l;
             split_d(kap * rg[r0 + q], h, l);
             kr[q] = make_float2(h, l);
@@ -485,11 +503,11 @@ __global__ void __launch_bounds__(kThreads, SER ? 2 : 3) fast_stage2(mma_hankel_
                 for (int i = 0; i < kSeriesPlanes; i++) As[i * rtile + q] = asel[((int64_t)i * No + o) * Nr + r0 + q];
         }
         __syncthreads();
-        if (threadIdx.x < (nt + kChunk - 1) / kChunk) {
-            const int64_t c0 = threadIdx.x * kChunk, c1 = c0 + kChunk < nt ? c0 + kChunk : nt;
-            float mx = 0.f;
-            for (int64_t q = c0; q < c1; q++) mx = fmaxf(mx, fabsf(kr[q].x));
-            s_krm[threadIdx.x] = mx * 1.000001f;  // k r / d_ref's low part and rounding: a hair above
+        for (int c = warp; c * kChunk < nt; c += kS2Threads / 32) {
+            const int q = c * kChunk + lane;
+            const float v = q < nt ? fmaxf(fabsf(kr[q].x), 0.f) : 0.f;
+            const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+            if (lane == 0) s_krm[c] = mx * 1.000001f;  // k r / d_ref's low part and rounding: a hair above
         }
         __syncthreads();
         if (j < Nrho) {
@@ -520,61 +538,79 @@ __global__ void __launch_bounds__(kThreads, SER ? 2 : 3) fast_stage2(mma_hankel_
                     cnt = 0;
                 }
             };
-            // radius pairs q, q + 1 in [qa, qb) with ML series terms
-            auto pairs = [&](auto MLc, int64_t qa, int64_t qb) {
-              constexpr int ML = decltype(MLc)::value;
-              for (int64_t q = qa; q + 1 < qb; q += 2) {
-                const float4 kk = kr4[q / 2];
-                const float2 kh = make_float2(kk.x, kk.z), kl = make_float2(kk.y, kk.w);
-                const float2 yh = __fmul2_rn(kh, f2b(rh));
-                const float2 yl = __fadd2_rn(__ffma2_rn(kh, f2b(rh), f2n(yh)), __ffma2_rn(kh, f2b(rl), __fmul2_rn(kl, f2b(rh))));
-                float2 J0, J1;
-                bessel01x2<true>(yh, yl, J0, J1);
-                const float2 y = __fadd2_rn(yh, yl);
-                float2 K0 = J0;
-                float2 K1 = __fmul2_rn(__fmul2_rn(f2b(0.5f * s), y), J1);
-                const float2 q2 = __fmul2_rn(__fmul2_rn(f2b(0.25f * s * s), y), y);
-                // lanes = the two radii throughout: the real and the imaginary parts of the far
-                // field's sum, and (SER) the planes' sums sum_m v_k0^m K_m and sum_m v_k1^m K_m
-                const float4 b0 = B4[q / 2], b1 = B4[rtile / 2 + q / 2];
-                float2 sre = __ffma2_rn(make_float2(b0.x, b0.y), K0, __fmul2_rn(make_float2(b1.x, b1.y), K1));
-                float2 sim = __ffma2_rn(make_float2(b0.z, b0.w), K0, __fmul2_rn(make_float2(b1.z, b1.w), K1));
-                float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+            // N radius pairs from radius q on, with ml series terms: the pairs share each broadcast
+            // constant, and their chains run interleaved
+            auto group = [&](auto Nc, int ml, int64_t q) {
+                constexpr int N = decltype(Nc)::value;
+                float2 yh[N], yl[N], K0[N], K1[N], q2[N], sre[N], sim[N], s0[N], s1[N];
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    const float4 kk = kr4[q / 2 + i];
+                    const float2 kh = make_float2(kk.x, kk.z), kl = make_float2(kk.y, kk.w);
+                    yh[i] = __fmul2_rn(kh, f2b(rh));
+                    const float2 e = __ffma2_rn(kh, f2b(-rh), yh[i]);  // minus the product's rounding error
+                    yl[i] = __ffma2_rn(e, f2b(-1.0f), __ffma2_rn(kh, f2b(rl), __fmul2_rn(kl, f2b(rh))));
+                }
+                bessel01n(yh, yl, K0, K1);
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    const float2 y = __fadd2_rn(yh[i], yl[i]);
+                    K1[i] = __fmul2_rn(__fmul2_rn(f2b(0.5f * s), y), K1[i]);
+                    q2[i] = __fmul2_rn(__fmul2_rn(f2b(0.25f * s * s), y), y);
+                    // lanes = the two radii throughout: the real and the imaginary parts of the far
+                    // field's sum, and (SER) the planes' sums sum_m v_k0^m K_m and sum_m v_k1^m K_m
+                    const float4 b0 = B4[q / 2 + i], b1 = B4[rtile / 2 + q / 2 + i];
+                    sre[i] = __ffma2_rn(make_float2(b0.x, b0.y), K0[i], __fmul2_rn(make_float2(b1.x, b1.y), K1[i]));
+                    sim[i] = __ffma2_rn(make_float2(b0.z, b0.w), K0[i], __fmul2_rn(make_float2(b1.z, b1.w), K1[i]));
+                    s0[i] = s1[i] = make_float2(0.f, 0.f);
+                }
                 if (SER) {
                     const float4 v = lds4(vb_s + 16u);
-                    s0 = __ffma2_rn(make_float2(v.x, v.y), K1, K0);  // v^0 = 1
-                    s1 = __ffma2_rn(make_float2(v.z, v.w), K1, K0);
+#pragma unroll
+                    for (int i = 0; i < N; i++) {
+                        s0[i] = __ffma2_rn(make_float2(v.x, v.y), K1[i], K0[i]);  // v^0 = 1
+                        s1[i] = __ffma2_rn(make_float2(v.z, v.w), K1[i], K0[i]);
+                    }
                 }
 #pragma unroll
-                for (int m = 1; m + 1 < ML; m++) {
-                    const float4 c = lds4(cm_s + 16u * m);
-                    const float2 K2 = __ffma2_rn(make_float2(c.x, c.y), K1,
-                                                 __fmul2_rn(__fmul2_rn(q2, make_float2(c.z, c.w)), K0));
-                    const float4 b = B4[(m + 1) * (rtile / 2) + q / 2];
-                    sre = __ffma2_rn(make_float2(b.x, b.y), K2, sre);
-                    sim = __ffma2_rn(make_float2(b.z, b.w), K2, sim);
+                for (int m = 1; m + 1 < MM; m++) {
+                    if ((MM > 8 && m + 1 == MM - 8 && ml == m + 1) || (MM > 4 && m + 1 == MM - 4 && ml == m + 1)) break;
+                    const float4 c = T.c[m];
+#pragma unroll
+                    for (int i = 0; i < N; i++) {
+                        const float2 K2 = __ffma2_rn(make_float2(c.x, c.y), K1[i],
+                                                     __fmul2_rn(__fmul2_rn(q2[i], make_float2(c.z, c.w)), K0[i]));
+                        const float4 b = B4[(m + 1) * (rtile / 2) + q / 2 + i];
+                        sre[i] = __ffma2_rn(make_float2(b.x, b.y), K2, sre[i]);
+                        sim[i] = __ffma2_rn(make_float2(b.z, b.w), K2, sim[i]);
+                        K0[i] = K1[i];
+                        K1[i] = K2;
+                    }
                     if (SER) {
                         const float4 v = lds4(vb_s + 16u * (m + 1));
-                        s0 = __ffma2_rn(make_float2(v.x, v.y), K2, s0);
-                        s1 = __ffma2_rn(make_float2(v.z, v.w), K2, s1);
+#pragma unroll
+                        for (int i = 0; i < N; i++) {
+                            s0[i] = __ffma2_rn(make_float2(v.x, v.y), K1[i], s0[i]);
+                            s1[i] = __ffma2_rn(make_float2(v.z, v.w), K1[i], s1[i]);
+                        }
                     }
-                    K0 = K1;
-                    K1 = K2;
                 }
-                add_in(make_float2(sre.x, sim.x), q, make_float2(s0.x, s1.x));
-                add_in(make_float2(sre.y, sim.y), q + 1, make_float2(s0.y, s1.y));
-              }
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    add_in(make_float2(sre[i].x, sim[i].x), q + 2 * i, make_float2(s0[i].x, s1[i].x));
+                    add_in(make_float2(sre[i].y, sim[i].y), q + 2 * i + 1, make_float2(s0[i].y, s1[i].y));
+                }
+            };
+            auto pairs = [&](int ml, int64_t qa, int64_t qb) {  // the radius pairs of [qa, qb)
+                int64_t q = qa;
+                for (; q + 2 * kS2Pairs <= qb; q += 2 * kS2Pairs) group(std::integral_constant<int, kS2Pairs>{}, ml, q);
+                for (; q + 1 < qb; q += 2) group(std::integral_constant<int, 1>{}, ml, q);
             };
             const float hs = 0.5f * s * rho_w;
             for (int64_t c0 = 0; c0 + 1 < nt; c0 += kChunk) {
                 const int64_t c1 = c0 + kChunk < nt ? c0 + kChunk : nt;
                 const float xc = hs * s_krm[c0 / kChunk];  // warp-uniform
-                if (MM > 8 && xc <= x_cut8)
-                    pairs(std::integral_constant<int, (MM > 8 ? MM - 8 : MM)>{}, c0, c1);
-                else if (MM > 4 && xc <= x_cut4)
-                    pairs(std::integral_constant<int, (MM > 4 ? MM - 4 : MM)>{}, c0, c1);
-                else
-                    pairs(std::integral_constant<int, MM>{}, c0, c1);
+                pairs(MM > 8 && xc <= x_cut8 ? MM - 8 : MM > 4 && xc <= x_cut4 ? MM - 4 : MM, c0, c1);
             }
             const int64_t q = nt - 1;
             if (nt & 1) {  // an odd last radius (all MM terms)
@@ -965,21 +1001,27 @@ int launch_fast(const mma_hankel_problem* p, const mma_hankel_fast_plan_t* plan,
     // stage 2: B, k r / d_ref and (series planes) their A_k rows per tile of rtile radii
     const int rows = MM + 1 + (ser ? kSeriesPlanes : 0);
     const size_t budget = (ser ? 72 : 96) * 1024;
-    const size_t consts = (ser ? MM * (sizeof(float2) + 2 * sizeof(float4)) : MM * sizeof(float4));
+    const size_t consts = ser ? MM * (sizeof(float2) + sizeof(float4)) : 0;
     int rtile = (int)(p->n_r < 512 ? p->n_r : 512);
     rtile += rtile & 1;  // even row stride: stage 2 loads radius pairs as 16-byte words
     while ((size_t)rows * rtile * sizeof(float2) + consts > budget && rtile > 32) rtile = (rtile / 2 + 1) & ~1;
     const size_t s2 = (size_t)rows * rtile * sizeof(float2) + consts;
-    dim3 g2((unsigned)((p->n_rho + kThreads - 1) / kThreads), (unsigned)p->n_omega);
+    dim3 g2((unsigned)((p->n_rho + kS2Threads - 1) / kS2Threads), (unsigned)p->n_omega);
     const float cut8 = series_cut(plan, MM - 8), cut4 = series_cut(plan, MM - 4);
+    stage2_terms<MM> T;
+    for (int m = 0; m < MM; m++) {
+        const float c1 = (float)plan->sigma * ((float)m / (float)(m + 1));
+        const float c2 = m > 0 ? -(1.0f / (float)(m * (m + 1))) : 0.f;
+        T.c[m] = make_float4(c1, c1, c2, c2);
+    }
     if (ser) {
         cudaFuncSetAttribute(fast_stage2<MM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
-        fast_stage2<MM, true><<<g2, kThreads, s2, st>>>(*p, *plan, og, rg, rho, Bp, ff, rtile, asel, vsel, n_sel,
-                                                         planes, cut8, cut4);
+        fast_stage2<MM, true><<<g2, kS2Threads, s2, st>>>(*p, *plan, og, rg, rho, Bp, ff, rtile, asel, vsel, n_sel,
+                                                         planes, cut8, cut4, T);
     } else {
         cudaFuncSetAttribute(fast_stage2<MM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
-        fast_stage2<MM, false><<<g2, kThreads, s2, st>>>(*p, *plan, og, rg, rho, Bp, ff, rtile, nullptr, nullptr, 0,
-                                                          nullptr, cut8, cut4);
+        fast_stage2<MM, false><<<g2, kS2Threads, s2, st>>>(*p, *plan, og, rg, rho, Bp, ff, rtile, nullptr, nullptr, 0,
+                                                          nullptr, cut8, cut4, T);
     }
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }

@@ -160,81 +160,89 @@ __device__ __forceinline__ void bessel01(float yh, float yl, float& J0, float& J
     }
 }
 
-// The same J0 and J1 for two arguments at once (x = (yh + yl).x and .y).  When both are >= 3 the
+// The same J0 and J1 for N pairs of arguments (x = (yh + yl).x and .y of each).  When all are >= 3 the
 // modulus/phase branch runs as packed FP32x2 instructions, each lane the operations of bessel01 in
-// the same order (the same bits); otherwise each lane takes bessel01.
+// the same order (the same bits; operands are negated through a constant, which costs no
+// instruction); otherwise each lane takes bessel01.  Coefficients are register pairs, and N pairs share
+// them.
 __device__ __forceinline__ float2 b2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 poly6(float2 t, float c6, float c5, float c4, float c3, float c2, float c1, float c0)
+template <int N, int D>
+__device__ __forceinline__ void poly_n(const float2 (&t)[N], const float (&c)[D], float2 (&f)[N])
 {
-    return __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, b2(c6), b2(c5)), b2(c4)),
-                                                              b2(c3)), b2(c2)), b2(c1)), b2(c0));
+#pragma unroll
+    for (int i = 0; i < N; i++) f[i] = b2(c[0]);
+#pragma unroll
+    for (int d = 1; d < D; d++)
+#pragma unroll
+        for (int i = 0; i < N; i++) f[i] = __ffma2_rn(t[i], f[i], b2(c[d]));
 }
-__device__ __forceinline__ float2 poly5(float2 t, float c5, float c4, float c3, float c2, float c1, float c0)
+#define MMA_EACH _Pragma("unroll") for (int i = 0; i < N; i++)
+template <int N>
+__device__ __forceinline__ void bessel01n(const float2 (&yh)[N], const float2 (&yl)[N], float2 (&J0)[N], float2 (&J1)[N])
 {
-    return __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, b2(c5), b2(c4)), b2(c3)), b2(c2)),
-                                    b2(c1)), b2(c0));
-}
-__device__ __forceinline__ void sincos_small2(float2 p, float2& s, float2& c)
-{
-    const float2 p2 = __fmul2_rn(p, p);
-    s = __fmul2_rn(p, __ffma2_rn(p2, __ffma2_rn(p2, b2(8.33333333e-3f), b2(-1.66666667e-1f)), b2(1.0f)));
-    c = __ffma2_rn(p2, __ffma2_rn(p2, b2(4.16666667e-2f), b2(-0.5f)), b2(1.0f));
-}
-template <bool WANT_J1>
-__device__ __forceinline__ void bessel01x2(float2 yh, float2 yl, float2& J0, float2& J1)
-{
-    if (!(yh.x >= 3.0f && yh.y >= 3.0f)) {
-        bessel01<WANT_J1>(yh.x, yl.x, J0.x, J1.x);
-        bessel01<WANT_J1>(yh.y, yl.y, J0.y, J1.y);
+    bool far = true;
+    MMA_EACH far = far && yh[i].x >= 3.0f && yh[i].y >= 3.0f;
+    if (!far) {
+        MMA_EACH {
+            bessel01<true>(yh[i].x, yl[i].x, J0[i].x, J1[i].x);
+            bessel01<true>(yh[i].y, yl[i].y, J0[i].y, J1[i].y);
+        }
         return;
     }
-    const float2 t = make_float2(__fdividef(3.0f, yh.x), __fdividef(3.0f, yh.y));
-    // reduce_2pi, lane by lane
-    const float2 kk = make_float2(rintf(yh.x * 0.159154943f), rintf(yh.y * 0.159154943f));
-    const float2 nk = make_float2(-kk.x, -kk.y);
-    float2 red = __ffma2_rn(nk, b2(6.28125f), yh);
-    red = __ffma2_rn(nk, b2(1.93500518798828125e-3f), red);
-    red = __ffma2_rn(nk, b2(3.0199159819370158e-07f), red);
-    red = __fadd2_rn(red, yl);
-    const float2 sq = make_float2(rsqrtf(yh.x), rsqrtf(yh.y));
-    // sincos_reduced, lane by lane
-    const float2 k = make_float2(rintf(red.x * 0.636619772f), rintf(red.y * 0.636619772f));
-    const float2 mk = make_float2(-k.x, -k.y);
-    float2 r = __ffma2_rn(mk, b2(1.5703125f), red);
-    r = __ffma2_rn(mk, b2(4.83826794896619e-4f), r);
-    const float2 r2 = __fmul2_rn(r, r);
-    const float2 ps = __fmul2_rn(
-        r, __ffma2_rn(r2, __ffma2_rn(r2, __ffma2_rn(r2, __ffma2_rn(r2, b2(2.75573192e-6f), b2(-1.98412698e-4f)),
-                                                    b2(8.33333333e-3f)), b2(-1.66666667e-1f)), b2(1.0f)));
-    const float2 pc = __ffma2_rn(r2, __ffma2_rn(r2, __ffma2_rn(r2, __ffma2_rn(r2, b2(2.48015873e-5f), b2(-1.38888889e-3f)),
-                                                              b2(4.16666667e-2f)), b2(-0.5f)), b2(1.0f));
-    float2 sr, cr;
+    float2 t[N], sq[N], r[N], a[N], b[N];
+    MMA_EACH t[i] = make_float2(__fdividef(3.0f, yh[i].x), __fdividef(3.0f, yh[i].y));
+    MMA_EACH sq[i] = make_float2(rsqrtf(yh[i].x), rsqrtf(yh[i].y));
     {
-        const int qx = (int)k.x & 3, qy = (int)k.y & 3;
-        const float ssx = (qx & 1) ? pc.x : ps.x, ccx = (qx & 1) ? ps.x : pc.x;
-        const float ssy = (qy & 1) ? pc.y : ps.y, ccy = (qy & 1) ? ps.y : pc.y;
-        sr = make_float2((qx & 2) ? -ssx : ssx, (qy & 2) ? -ssy : ssy);
-        cr = make_float2(((qx + 1) & 2) ? -ccx : ccx, ((qy + 1) & 2) ? -ccy : ccy);
+        // reduce_2pi, lane by lane
+        float2 k[N];
+        MMA_EACH k[i] = __fmul2_rn(yh[i], b2(0.159154943f));
+        MMA_EACH k[i] = make_float2(rintf(k[i].x), rintf(k[i].y));
+        MMA_EACH r[i] = __ffma2_rn(k[i], b2(-6.28125f), yh[i]);
+        MMA_EACH r[i] = __ffma2_rn(k[i], b2(-1.93500518798828125e-3f), r[i]);
+        MMA_EACH r[i] = __ffma2_rn(k[i], b2(-3.0199159819370158e-07f), r[i]);
+        MMA_EACH r[i] = __fadd2_rn(r[i], yl[i]);
+        // sincos_reduced, lane by lane
+        MMA_EACH k[i] = __fmul2_rn(r[i], b2(0.636619772f));
+        MMA_EACH k[i] = make_float2(rintf(k[i].x), rintf(k[i].y));
+        MMA_EACH r[i] = __ffma2_rn(k[i], b2(-1.5703125f), r[i]);
+        MMA_EACH r[i] = __ffma2_rn(k[i], b2(-4.83826794896619e-4f), r[i]);
+        float2 r2[N], ps[N], pc[N];
+        MMA_EACH r2[i] = __fmul2_rn(r[i], r[i]);
+        poly_n(r2, {2.75573192e-6f, -1.98412698e-4f, 8.33333333e-3f, -1.66666667e-1f, 1.0f}, ps);
+        poly_n(r2, {2.48015873e-5f, -1.38888889e-3f, 4.16666667e-2f, -0.5f, 1.0f}, pc);
+        MMA_EACH ps[i] = __fmul2_rn(r[i], ps[i]);
+        float2 sr[N], cr[N];
+        MMA_EACH {
+            const int qx = (int)k[i].x & 3, qy = (int)k[i].y & 3;
+            const float ssx = (qx & 1) ? pc[i].x : ps[i].x, ccx = (qx & 1) ? ps[i].x : pc[i].x;
+            const float ssy = (qy & 1) ? pc[i].y : ps[i].y, ccy = (qy & 1) ? ps[i].y : pc[i].y;
+            sr[i] = make_float2((qx & 2) ? -ssx : ssx, (qy & 2) ? -ssy : ssy);
+            cr[i] = make_float2(((qx + 1) & 2) ? -ccx : ccx, ((qy + 1) & 2) ? -ccy : ccy);
+        }
+        MMA_EACH a[i] = __fadd2_rn(cr[i], sr[i]);
+        MMA_EACH b[i] = __ffma2_rn(sr[i], b2(-1.0f), cr[i]);
     }
-    const float2 a = __fadd2_rn(cr, sr), b = __fadd2_rn(cr, make_float2(-sr.x, -sr.y));
-    const float2 f0 = poly6(t, 0.00014476f, -0.00072805f, 0.00137237f, -0.00009512f, -0.00552740f, -0.00000077f,
-                            0.79788456f);
-    const float2 p0 = __fmul2_rn(t, poly5(t, 0.00013558f, -0.00029333f, -0.00054125f, 0.00262573f, -0.00003954f,
-                                          -0.04166397f));
-    float2 s0, c0;
-    sincos_small2(p0, s0, c0);
-    J0 = __fmul2_rn(__fmul2_rn(f0, sq), __fmul2_rn(b2(0.707106781f), __ffma2_rn(c0, a, __fmul2_rn(s0, b))));
-    if (WANT_J1) {
-        const float2 f1 = poly6(t, -0.00020033f, 0.00113653f, -0.00249511f, 0.00017105f, 0.01659667f, 0.00000156f,
-                                0.79788456f);
-        const float2 p1 = __fmul2_rn(t, poly5(t, -0.00029166f, 0.00079824f, 0.00074348f, -0.00637879f, 0.00005650f,
-                                              0.12499612f));
-        float2 s1, c1;
-        sincos_small2(p1, s1, c1);
-        const float2 cb = __fmul2_rn(c1, b);
-        J1 = __fmul2_rn(__fmul2_rn(f1, sq), __fmul2_rn(b2(0.707106781f), __ffma2_rn(s1, a, make_float2(-cb.x, -cb.y))));
-    }
+    float2 f[N], p[N], p2[N], s[N], c[N];
+    poly_n(t, {0.00014476f, -0.00072805f, 0.00137237f, -0.00009512f, -0.00552740f, -0.00000077f, 0.79788456f}, f);
+    poly_n(t, {0.00013558f, -0.00029333f, -0.00054125f, 0.00262573f, -0.00003954f, -0.04166397f}, p);
+    MMA_EACH p[i] = __fmul2_rn(t[i], p[i]);
+    MMA_EACH p2[i] = __fmul2_rn(p[i], p[i]);
+    poly_n(p2, {8.33333333e-3f, -1.66666667e-1f, 1.0f}, s);  // sincos_small
+    MMA_EACH s[i] = __fmul2_rn(p[i], s[i]);
+    poly_n(p2, {4.16666667e-2f, -0.5f, 1.0f}, c);
+    MMA_EACH J0[i] = __fmul2_rn(__fmul2_rn(f[i], sq[i]),
+                                __fmul2_rn(b2(0.707106781f), __ffma2_rn(c[i], a[i], __fmul2_rn(s[i], b[i]))));
+    poly_n(t, {-0.00020033f, 0.00113653f, -0.00249511f, 0.00017105f, 0.01659667f, 0.00000156f, 0.79788456f}, f);
+    poly_n(t, {-0.00029166f, 0.00079824f, 0.00074348f, -0.00637879f, 0.00005650f, 0.12499612f}, p);
+    MMA_EACH p[i] = __fmul2_rn(t[i], p[i]);
+    MMA_EACH p2[i] = __fmul2_rn(p[i], p[i]);
+    poly_n(p2, {8.33333333e-3f, -1.66666667e-1f, 1.0f}, s);
+    MMA_EACH s[i] = __fmul2_rn(p[i], s[i]);
+    poly_n(p2, {-4.16666667e-2f, 0.5f, -1.0f}, c);  // -cos
+    MMA_EACH J1[i] = __fmul2_rn(__fmul2_rn(f[i], sq[i]),
+                                __fmul2_rn(b2(0.707106781f), __ffma2_rn(s[i], a[i], __fmul2_rn(c[i], b[i]))));
 }
+#undef MMA_EACH
 
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e)
 {

@@ -270,8 +270,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             const float2 rh = make_float2(rv.x, rv.z), rl = make_float2(rv.y, rv.w);
             const float2 yh = __fmul2_rn(bc2(kh), rh);
             const float2 yl = __fadd2_rn(__ffma2_rn(bc2(kh), rh, neg2(yh)), __ffma2_rn(bc2(kh), rl, __fmul2_rn(bc2(kl), rh)));
-            float2 J0, J1;
-            bessel01x2<true>(yh, yl, J0, J1);
+            const float2 yhs[1] = {yh}, yls[1] = {yl};
+            float2 J0s[1], J1s[1];
+            bessel01n(yhs, yls, J0s, J1s);
+            const float2 J0 = J0s[0], J1 = J1s[0];
             // K^_m = u^m J_m(y), u = y / y_max <= 1:  K^_{m+1} = (2m / y_max) K^_m - u^2 K^_{m-1}
             const float2 u = __fmul2_rn(__fadd2_rn(yh, yl), bc2(iy));
             const float2 w = __fmul2_rn(u, u);
