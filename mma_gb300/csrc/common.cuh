@@ -27,10 +27,12 @@ __device__ __forceinline__ cd cfms(cd b, cd c, cd a)
 {
     return cd{fma(-b.re, c.re, fma(b.im, c.im, a.re)), fma(-b.re, c.im, fma(-b.im, c.re, a.im))};
 }
+// fused operations spelled out: which product of a sum is fused decides the last bit, and with it the
+// rounding of everything that complex64 propagation makes of the tables
 __device__ __forceinline__ cd cdiv(cd a, cd b)
 {
-    double d = b.re * b.re + b.im * b.im;
-    return cd{(a.re * b.re + a.im * b.im) / d, (a.im * b.re - a.re * b.im) / d};
+    const double d = fma(b.re, b.re, b.im * b.im);
+    return cd{fma(a.re, b.re, a.im * b.im) / d, fma(a.im, b.re, -(a.re * b.im)) / d};
 }
 __device__ __forceinline__ cd ld2(const double* p) { double2 v = *reinterpret_cast<const double2*>(p); return cd{v.x, v.y}; }
 __device__ __forceinline__ void st2(double* p, cd v) { *reinterpret_cast<double2*>(p) = make_double2(v.re, v.im); }

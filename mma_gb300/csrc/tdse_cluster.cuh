@@ -72,19 +72,6 @@ struct Fp64 {
     };
 };
 
-// real FP64 (the ground state): what the scans need
-struct Real64 {
-    typedef double C;
-    static __device__ C zero() { return 0.0; }
-    static __device__ C one() { return 1.0; }
-    static __device__ bool tiny(C a) { return fabs(a) < kTiny; }
-    static __device__ C mul(C a, C b) { return a * b; }
-    static __device__ C fma(C a, C b, C z) { return ::fma(a, b, z); }
-    static __device__ C shup(C v, int d) { return shfl_up(v, d); }
-    static __device__ C shdn(C v, int d) { return shfl_down(v, d); }
-    static __device__ C bcast(C v, int l) { return shfl_idx(v, l); }
-};
-
 struct Df64 {
     typedef dfk::pk C;
     typedef dfk::df R;

@@ -24,8 +24,8 @@ int launch_cluster(const ClusterPlan& p, const mma_tdse_instance* insts, int n_i
 
 // The ground states of a few grids by a cluster each, from the tables and V that build_grids_kernel mode 3
 // left; false (and nothing launched) where a CTA per grid serves better (tdse_ground.cu).
-bool ground_state_cluster(const mma_tdse_grid* grids_dev, int n_grids, int64_t max_n, int sms, cudaStream_t st);
+bool ground_state_cluster(const mma_tdse_grid* grids_dev, int n_grids, int64_t max_m, int sms, cudaStream_t st);
 // x and the ground state of one grid, without its Crank-Nicolson tables (tdse_kernels.cu)
-int ground_state_only(const mma_tdse_grid* grid_dev, int64_t n, cudaStream_t st);
+int ground_state_only(const mma_tdse_grid* grid_dev, int64_t m, cudaStream_t st);
 
 }  // namespace mma

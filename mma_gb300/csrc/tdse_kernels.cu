@@ -31,9 +31,10 @@ namespace mma {
 // The pivots beta_j = b_j - a_j c_{j-1} / beta_{j-1} are a chain of Moebius maps, beta = p/q with
 // (p, q) -> (b_j p - e_j q, p), e_j = a_j c_{j-1}.  Each thread multiplies the 2x2 matrices of its m
 // sites (rescaled by powers of two), a CTA scan composes them, and the thread then runs the plain
-// recurrence over its chunk from the pivot just before it.  One thread running the whole chain took
-// 10 ms for 8001 sites (dependent FP64 divisions), 18 ms with the complex matrix of the step; split
-// over 256 threads the two take 0.1 ms.
+// recurrence over its chunk from the pivot just before it, again and again until the chunks agree to
+// the bit (see below).  One thread running the whole chain took 10 ms for 8001 sites (dependent FP64
+// divisions), 18 ms with the complex matrix of the step; split over 256 threads they take 0.3 and
+// 0.4 ms.
 // ------------------------------------------------------------------------------------------
 template <typename T>
 struct Moebius {
@@ -45,12 +46,10 @@ __device__ __forceinline__ double scale_(double v, double s) { return v * s; }
 __device__ __forceinline__ cd scale_(cd v, double s) { return cd{v.re * s, v.im * s}; }
 __device__ __forceinline__ double neg_(double v) { return -v; }
 __device__ __forceinline__ cd neg_(cd v) { return cd{-v.re, -v.im}; }
-__device__ __forceinline__ double inv_(double v) { return 1.0 / v; }
-__device__ __forceinline__ cd inv_(cd v)
-{
-    const double s = 1.0 / fma(v.re, v.re, v.im * v.im);
-    return cd{v.re * s, -v.im * s};
-}
+__device__ __forceinline__ double div_(double a, double b) { return a / b; }
+__device__ __forceinline__ cd div_(cd a, cd b) { return cdiv(a, b); }
+__device__ __forceinline__ bool same_(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
+__device__ __forceinline__ bool same_(cd a, cd b) { return same_(a.re, b.re) && same_(a.im, b.im); }
 
 template <typename T>
 __device__ __forceinline__ void rescale(Moebius<T>& M)
@@ -71,9 +70,9 @@ __device__ __forceinline__ Moebius<T> compose(const Moebius<T>& B, const Moebius
     return M;
 }
 
-// `warp`: kWarps entries of shared scratch.  Contains __syncthreads.
+// `warp` and `ends`: kWarps and kThreads entries of shared scratch.  Contains __syncthreads.
 template <typename T, typename RowFn>
-__device__ void factorise(int64_t n, int64_t m, T* ib, T* h, T* g, double rhs_scale, Moebius<T>* warp, RowFn row)
+__device__ void factorise(int64_t n, int64_t m, T* ib, T* h, T* g, double rhs_scale, Moebius<T>* warp, T* ends, RowFn row)
 {
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     T one;
@@ -116,20 +115,41 @@ __device__ void factorise(int64_t n, int64_t m, T* ib, T* h, T* g, double rhs_sc
         p = pn;
         q = qn;
     }
-    T ibeta = (j0 > 0 && j0 < n) ? mul_(q, inv_(p)) : zero;  // 1 / beta_{j0 - 1}
-    for (int64_t j = j0; j < j1; j++) {
-        row(j, a, b, c);
-        T beta = b;
-        if (j > 0) {
-            // gamma_{j-1} = c_{j-1} / beta_{j-1}; beta_j = b_j - a_j gamma_{j-1}
-            const T gam = mul_(cprev, ibeta);
-            g[qidx(j - 1, m)] = gam;
-            beta = axpy_(neg_(a), gam, b);
+    // The chain from there on, with the operations of a serial run.  Its own pivots differ from the
+    // composed ones in the last digits, but a pivot forgets its start within a few sites: a chunk whose
+    // start is not the value the chunk before ended on runs again from that value, until all agree.
+    // Chunk 0 is exact and each round makes the next one final, so it ends, and on the serial bits.
+    T start = (j0 > 0 && j0 < n) ? div_(p, q) : zero;
+    bool run = j0 < n;
+    for (;;) {
+        if (run) {
+            T beta = start;
+            cp = cprev;
+            for (int64_t j = j0; j < j1; j++) {
+                row(j, a, b, c);
+                if (j > 0) {
+                    // gamma_{j-1} = c_{j-1} / beta_{j-1}; beta_j = b_j - a_j gamma_{j-1}
+                    const T gam = div_(cp, beta);
+                    g[qidx(j - 1, m)] = gam;
+                    beta = b - mul_(a, gam);
+                } else {
+                    beta = b;
+                }
+                const T ibeta = div_(one, beta);
+                ib[qidx(j, m)] = scale_(ibeta, rhs_scale);
+                h[qidx(j, m)] = (j > 0) ? mul_(a, ibeta) : zero;
+                cp = c;
+            }
+            ends[t] = beta;
         }
-        ibeta = inv_(beta);
-        ib[qidx(j, m)] = scale_(ibeta, rhs_scale);
-        h[qidx(j, m)] = (j > 0) ? mul_(a, ibeta) : zero;
-        cprev = c;
+        __syncthreads();
+        run = false;
+        if (t > 0 && j0 < n) {
+            const T e = ends[t - 1];
+            run = !same_(e, start);
+            start = e;
+        }
+        if (!__syncthreads_or(run)) break;
     }
     if (t == 0) g[qidx(n - 1, m)] = zero;
     __syncthreads();
@@ -233,8 +253,8 @@ __device__ void ground_state(const mma_tdse_grid& G, const double* tab, double* 
             int64_t q = i * kThreads + t;
             double pn = (i + 1 < m) ? psi[q + kThreads] : ((t + 1 < kThreads) ? psi[t + 1] : 0.0);
             double vn = (i + 1 < m) ? vq[q + kThreads] : ((t + 1 < kThreads) ? vq[t + 1] : 0.0);
-            double kpsi = inv_dx2 * pc - 0.5 * inv_dx2 * (pm + pn) + (10.0 / 12.0) * pc * vc + (pm * vm + pn * vn) / 12.0;
-            double mpsi = 10.0 * pc / 12.0 + (pm + pn) / 12.0;
+            double kpsi, mpsi;
+            quotient_terms(inv_dx2, pm, pc, pn, vm, vc, vn, (int)i, (int)m, kpsi, mpsi);
             if (t * m + i < n) {  // the row past the grid's end sees psi_{n-1} too, but is no row of the quotient
                 acc[0] = fma(kpsi, mpsi, acc[0]);
                 acc[1] = fma(mpsi, mpsi, acc[1]);
@@ -288,7 +308,9 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
     __shared__ double red[kWarps * 4];
     __shared__ double sc[2 * kWarps], sb[2 * kWarps];
     __shared__ Moebius<cd> maps[kWarps];
+    __shared__ cd ends[kThreads];
     Moebius<double>* const rmaps = reinterpret_cast<Moebius<double>*>(maps);
+    double* const rends = reinterpret_cast<double*>(ends);
     const mma_tdse_grid G = grids[blockIdx.x];
     const int t = threadIdx.x;
     const int64_t n = G.n, m = G.m, L = m * kThreads, num_r = n - 1;
@@ -318,7 +340,7 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
                 bj = 10.0 * vj / 12.0 + d0 - 10.0 * E / 12.0;
                 cj = (j + 1 < n) ? k0 - E / 12.0 + V[j + 1] / 12.0 : 0.0;
             };
-            factorise<double>(n, m, gtab + GS_IB12 * L, gtab + GS_H * L, gtab + GS_G * L, 1.0 / 12.0, rmaps, row);
+            factorise<double>(n, m, gtab + GS_IB12 * L, gtab + GS_H * L, gtab + GS_G * L, 1.0 / 12.0, rmaps, rends, row);
         }
         chunk_products<double>(m, gtab + GS_H * L, gtab + GS_G * L, gtab + GS_F * L, gtab + GS_GG * L);
         __syncthreads();
@@ -344,7 +366,7 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
             bj = cd{10.0 / 12.0, hdt * (1.0 / (dx * dx)) + hdt * 10 / 12. * vj};
             cj = (j + 1 < n) ? cd{1.0 / 12.0, hdt * (-0.5 / (dx * dx)) + hdt * 1 / 12. * V[j + 1]} : cd{0.0, 0.0};
         };
-        factorise<cd>(n, m, ctab + CN_IB6 * L, ctab + CN_H * L, ctab + CN_G * L, 1.0 / 6.0, maps, row);
+        factorise<cd>(n, m, ctab + CN_IB6 * L, ctab + CN_H * L, ctab + CN_G * L, 1.0 / 6.0, maps, ends, row);
     }
     chunk_products<cd>(m, ctab + CN_H * L, ctab + CN_G * L, ctab + CN_F * L, ctab + CN_GG * L);
     __syncthreads();
@@ -362,7 +384,7 @@ __global__ void __launch_bounds__(kThreads) build_grids_kernel(const mma_tdse_gr
                 bj = cd{10.0 / 12.0, -(hdt * (1.0 / (dx * dx)) + hdt * 10 / 12. * V[j])};
                 cj = (j + 1 < n) ? cd{1.0 / 12.0, -wj} : cd{0.0, 0.0};
             };
-            factorise<cd>(n, m, atab + CN_IB6 * L, atab + CN_H * L, atab + CN_G * L, 1.0, maps, row);
+            factorise<cd>(n, m, atab + CN_IB6 * L, atab + CN_H * L, atab + CN_G * L, 1.0, maps, ends, row);
         }
         chunk_products<cd>(m, atab + CN_H * L, atab + CN_G * L, atab + CN_F * L, atab + CN_GG * L);
         __syncthreads();
@@ -577,17 +599,17 @@ static int sm_count()
 }
 
 // x and the ground states of grids with their tables: by a cluster per grid where they are few
-static bool few_ground_states(const mma_tdse_grid* grids_dev, int n_grids, int64_t max_n, cudaStream_t st)
+static bool few_ground_states(const mma_tdse_grid* grids_dev, int n_grids, int64_t max_m, cudaStream_t st)
 {
     const int sms = sm_count();
     if (n_grids * 4 > sms) return false;
     build_grids_kernel<<<n_grids, kThreads, 0, st>>>(grids_dev, 3);
-    return ground_state_cluster(grids_dev, n_grids, max_n, sms, st);
+    return ground_state_cluster(grids_dev, n_grids, max_m, sms, st);
 }
 
-int mma::ground_state_only(const mma_tdse_grid* grid_dev, int64_t n, cudaStream_t st)
+int mma::ground_state_only(const mma_tdse_grid* grid_dev, int64_t m, cudaStream_t st)
 {
-    if (!few_ground_states(grid_dev, 1, n, st)) build_grids_kernel<<<1, kThreads, 0, st>>>(grid_dev, 2);
+    if (!few_ground_states(grid_dev, 1, m, st)) build_grids_kernel<<<1, kThreads, 0, st>>>(grid_dev, 2);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }
 
@@ -602,9 +624,9 @@ extern "C" int mma_tdse_build_grids(const mma_tdse_grid* grids_dev, const mma_td
             return MMA_ERR_ARG;
         if (mode == 0 && G.max_iter < 1) return MMA_ERR_ARG;
     }
-    int64_t max_n = 0;
-    for (int g = 0; g < n_grids; g++) max_n = grids_host[g].n > max_n ? grids_host[g].n : max_n;
-    if (mode == 0 && few_ground_states(grids_dev, n_grids, max_n, (cudaStream_t)stream)) mode = 1;
+    int64_t max_m = 0;
+    for (int g = 0; g < n_grids; g++) max_m = grids_host[g].m > max_m ? grids_host[g].m : max_m;
+    if (mode == 0 && few_ground_states(grids_dev, n_grids, max_m, (cudaStream_t)stream)) mode = 1;
     build_grids_kernel<<<n_grids, kThreads, 0, (cudaStream_t)stream>>>(grids_dev, mode);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }

@@ -134,7 +134,7 @@ extern "C" void Initialise_grid_and_ground_state(inputs_def* in)
         free_grid(g);
         return;
     }
-    rc = mma::ground_state_only(g.d, n, nullptr);  // call1DTDSE builds the step's tables for its own dt
+    rc = mma::ground_state_only(g.d, g.h.m, nullptr);  // call1DTDSE builds the step's tables for its own dt
     if (rc != MMA_OK) {
         set_status(rc, "grid build launch failed");
         free_grid(g);

@@ -21,6 +21,20 @@ __device__ __forceinline__ double minus_grad_v(double x, double a)
     return x / (s * sqrt(s));
 }
 
+// (K psi) and (M2 psi) at site i of a thread's m in the energy quotient (tridiag.c:172-238).  The inverse
+// iteration stops on this quotient's rounding, so its last bit decides how often it runs and with that
+// psi0's twelfth digit: every fused operation is spelled out.  Which of the neighbours' two products is
+// fused alternates by pairs of sites, as it always has.
+__device__ __forceinline__ void quotient_terms(double inv_dx2, double pm, double pc, double pn, double vm, double vc,
+                                               double vn, int i, int m, double& kpsi, double& mpsi)
+{
+    const double kin = fma(inv_dx2, pc, -(0.5 * inv_dx2 * (pm + pn)));
+    const bool right = (i & 2) && i < (m & ~3);
+    const double nb = right ? fma(pn, vn, pm * vm) : fma(pm, vm, pn * vn);
+    kpsi = fma((10.0 / 12.0) * pc, vc, kin) + nb / 12.0;
+    mpsi = 10.0 * pc / 12.0 + (pm + pn) / 12.0;
+}
+
 __device__ __forceinline__ int64_t qidx(int64_t j, int64_t m) { return (j % m) * kThreads + (j / m); }
 
 // First index where the reference's zero gate opens: the first k with f[k] f[k+1] <= 0

@@ -175,3 +175,18 @@ def test_ground_state_cluster_iteration_cap(gpu_lib):
 
     with pytest.raises(MMAStatusError, match="not converged"):
         TDSEGrids([dict(num_r=600, dx=0.4, trg_a=A_CONFIG, max_iter=3)], dt=0.25)
+
+
+@pytest.mark.parametrize("num_r,dx", [(255, 0.4), (256, 0.4), (777, 0.2), (1023, 0.1), (2400, 0.2), (8000, 0.1)])
+def test_few_grids_and_many_give_the_same_bits(gpu_lib, num_r, dx):
+    """One grid (a cluster per grid) against the same grid among as many as a CTA each serves: ground
+    state, energy, iterations and tables are the same bits, since both run the same operations."""
+    import torch
+    from mma_gb300.tdse_batch import TDSEGrids
+
+    p = dict(num_r=num_r, dx=dx, trg_a=A_CONFIG)
+    one = TDSEGrids([p], dt=0.25)
+    many = TDSEGrids([p] * (torch.cuda.get_device_properties(0).multi_processor_count // 4 + 1), dt=0.25)
+    for name in ("x", "psi0", "cn_tab", "gs_tab", "result"):
+        (o, cnt), (q, _) = one.views[0][name], many.views[-1][name]
+        assert torch.equal(one.buf[o:o + cnt].view(torch.int64), many.buf[q:q + cnt].view(torch.int64)), name

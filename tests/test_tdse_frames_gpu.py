@@ -26,7 +26,7 @@ def test_frames_match_fp64(gpu_lib, num_r, dx, n_f):
     from mma_gb300.tdse_batch import TDSEGrids, run_batch
 
     fields = _fields(n_f, 2)
-    grids = TDSEGrids([dict(num_r=num_r, dx=dx, trg_a=A_CONFIG, max_iter=100000)], dt=0.25, df64=True)
+    grids = TDSEGrids([dict(num_r=num_r, dx=dx, trg_a=A_CONFIG, CV=1e-13)], dt=0.25, df64=True)
     got, ref = (run_batch(grids, fields, 0.25, precision=p, psi_final=True, snap_every=7, grid_ctas=1)
                 for p in ("df64", "fp64"))
     torch.cuda.synchronize()
