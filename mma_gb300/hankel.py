@@ -397,14 +397,16 @@ def _uniform_tables_on_device(z, w, dev, pressure, want_renorm, **medium):
     disp, absorb = _uniform_medium(w, pressure=pressure, **medium)
     if np.iscomplexobj(disp) or np.iscomplexobj(absorb):
         return None
-    pre = torch.empty(len(z), len(w), dtype=torch.complex128, device=dev)
-    renorm = torch.empty(len(z), len(w), dtype=torch.float64, device=dev) if want_renorm else None
-    zd, wd, dd, ad = (_dev(a, dev) for a in (z, w, np.broadcast_to(disp, w.shape), np.broadcast_to(absorb, w.shape)))
-    _check(_sig().mma_hankel_uniform_pre_factor(len(z), len(w), zd.data_ptr(), wd.data_ptr(), dd.data_ptr(),
-                                                ad.data_ptr(), float(pressure), pre.data_ptr(),
-                                                None if renorm is None else renorm.data_ptr(),
-                                                ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)),
-           "mma_hankel_uniform_pre_factor")
+    with torch.cuda.device(dev):  # the kernel runs on the source's device, whichever is current
+        pre = torch.empty(len(z), len(w), dtype=torch.complex128, device=dev)
+        renorm = torch.empty(len(z), len(w), dtype=torch.float64, device=dev) if want_renorm else None
+        zd, wd, dd, ad = (_dev(a, dev) for a in (z, w, np.broadcast_to(disp, w.shape),
+                                                 np.broadcast_to(absorb, w.shape)))
+        _check(_sig().mma_hankel_uniform_pre_factor(len(z), len(w), zd.data_ptr(), wd.data_ptr(), dd.data_ptr(),
+                                                    ad.data_ptr(), float(pressure), pre.data_ptr(),
+                                                    None if renorm is None else renorm.data_ptr(),
+                                                    ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)),
+               "mma_hankel_uniform_pre_factor")
     return pre, renorm
 
 
@@ -816,17 +818,18 @@ def _cumulative(z, planes, renorm, want_running):
     renormalisation table, renorm_factor(k1) times it (:640-672; row k1, not k1 + 1, as in :668)."""
     Nz, (nrho, no), dev = len(z), planes[0].shape, planes[0].device
     step = planes[0].numel() * planes[0].element_size()
-    if not all(p.is_contiguous() and p.data_ptr() == planes[0].data_ptr() + k * step for k, p in enumerate(planes)):
-        planes = list(torch.stack(planes))  # planes of separate allocations
-    empty = lambda: torch.empty(Nz - 1, nrho, no, dtype=torch.complex128, device=dev)  # noqa: E731
-    norm, run = None if renorm is None else empty(), empty() if want_running else None
-    prob = HankelProblem(no, 2, Nz, nrho, 1.0, 0, 1, 0, 2, 0)  # only n_z, n_rho and n_omega count
-    zd = _dev(z, dev)
-    rn = None if renorm is None else _dev(renorm, dev)
-    ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
-    _check(_sig().mma_hankel_cumulative(ctypes.byref(prob), zd.data_ptr(), planes[0].data_ptr(), ptr(rn), ptr(norm),
-                                        ptr(run), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)),
-           "mma_hankel_cumulative")
+    with torch.cuda.device(dev):  # the kernel runs on the planes' device, whichever is current
+        if not all(p.is_contiguous() and p.data_ptr() == planes[0].data_ptr() + k * step for k, p in enumerate(planes)):
+            planes = list(torch.stack(planes))  # planes of separate allocations
+        empty = lambda: torch.empty(Nz - 1, nrho, no, dtype=torch.complex128, device=dev)  # noqa: E731
+        norm, run = None if renorm is None else empty(), empty() if want_running else None
+        prob = HankelProblem(no, 2, Nz, nrho, 1.0, 0, 1, 0, 2, 0)  # only n_z, n_rho and n_omega count
+        zd = _dev(z, dev)
+        rn = None if renorm is None else _dev(renorm, dev)
+        ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+        _check(_sig().mma_hankel_cumulative(ctypes.byref(prob), zd.data_ptr(), planes[0].data_ptr(), ptr(rn), ptr(norm),
+                                            ptr(run), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)),
+               "mma_hankel_cumulative")
     return norm, run
 
 
