@@ -226,6 +226,7 @@ struct ClusterArgs {
 };
 
 constexpr int kGradRing = 8;
+static_assert(4 * kGradRing == 32, "one warp sums the collected steps");
 
 __host__ __device__ inline size_t adj_site_bytes() { return 6 * 16; }
 __host__ __device__ inline size_t adj_fixed_bytes(int nc)
@@ -357,13 +358,14 @@ __global__ void __launch_bounds__(clk::kT, 1) adjoint_cluster_kernel(ClusterArgs
         for (int i = 0; i < m; i++) lam[i * kT + t] = N::zero();  // lambda_S = 0
         // rank 0: the gradient of steps k, k - 1, ... (cnt of them) from ring slots slot0, slot0 + 1, ...
         auto flush = [&](int64_t k, int cnt) {
-            if (t < 4 * cnt) {
-                const int sl = t / 4;
+            if (w == 0) {  // four lanes a step; the whole warp shuffles
+                const int sl = lane / 4;
                 double s = 0.0;
-                for (int q = t % 4; q < NW; q += 4) s += ring[sl * NW + q];
-                s += __shfl_xor_sync(__activemask(), s, 1);
-                s += __shfl_xor_sync(__activemask(), s, 2);
-                if (t % 4 == 0) gi[k - sl] = ai[k - sl + 1] - dt * s;
+                if (sl < cnt)
+                    for (int q = lane % 4; q < NW; q += 4) s += ring[sl * NW + q];
+                s += shfl_xor(s, 1);
+                s += shfl_xor(s, 2);
+                if (sl < cnt && lane % 4 == 0) gi[k - sl] = ai[k - sl + 1] - dt * s;
             }
         };
 
