@@ -386,6 +386,22 @@ int pes_sms()
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return sms > 0 ? sms : 1;
 }
+
+// Whether pairs serve `left` energies (or the first wave of them, 64 energies an SM) of n rows sooner than a
+// warp each.  Pairs take a chain of n/2 rows twice, however many they are; a warp each has 1/32 of the chain
+// but 66 operations a row against 40 and, per energy, two cyclic reductions across its lanes, as much as six
+// rows a lane.  us, measured / model: pairs 51 rows 77 / 88, 601 rows 980 / 979, 8001 rows 13000 / 12970;
+// warps 51 rows, 3000 energies 188 / 167, 601 rows, 10 energies 112 / 109, 3000 energies 620 / 637, 8001
+// rows, 50 energies 1370 / 1340, 3000 energies 7040 / 7040, 5000 energies 11000 / 11030.  (One thread an
+// energy took 26 to 34 ms for 8001 rows; 10000 energies take 13.9 ms, a wave of pairs and 272 warps.)
+bool pes_by_pairs(int64_t left, int64_t n, int sms)
+{
+    if (n < 4) return false;
+    if (left >= (int64_t)64 * sms) return true;
+    const double m = (double)((n + 31) / 32), chain = 8.0 + 5.3 * m;
+    const double load = 0.8 * chain + (double)left * (0.035 + 0.0078 * m) * 152.0 / sms;
+    return 5.0 + 1.62 * (double)n < (chain > load ? chain : load);
+}
 }  // namespace
 
 extern "C" size_t mma_tdse_pes_scratch_bytes(int num_r, int chunk)
@@ -394,7 +410,8 @@ extern "C" size_t mma_tdse_pes_scratch_bytes(int num_r, int chunk)
     const size_t n = (size_t)num_r + 1, m = (n + 31) / 32;
     // the pairs' two arrays of `chunk` energies, then gamma, y and f of the energies that a warp each
     // takes: those beyond full waves of pairs, as many as run at once (16 warps an SM)
-    const size_t wave = 64 * 152, rest = (size_t)chunk % wave * 5 > wave * 3 ? 0 : (size_t)chunk % wave;
+    const size_t wave = 64 * 152, left = (size_t)chunk % wave;
+    const size_t rest = left > 0 && !pes_by_pairs((int64_t)left, (int64_t)n, 152) ? left : 0;
     const size_t warps = ((size_t)chunk < wave ? (size_t)chunk : rest) + 3;
     return pes_fixed(n) + 32 * m * 24 + 512 + 2 * sizeof(cd) * n * ((size_t)chunk - rest) +
            48 * 32 * m * ((warps < 16 * 152 ? warps : 16 * 152) / 4 * 4);
@@ -426,15 +443,16 @@ extern "C" int mma_tdse_pes(const double* psi, int num_r, double dx, double trg_
     cd* buf = reinterpret_cast<cd*>(rest + tabs);
     room -= tabs;
     an::pes_tables<<<an::grid_for(32 * m), 256, 0, st>>>(n, m, num_r, dx, trg_a, psi, V12, rhs0, V12t, rhs0t);
-    // full waves of pairs (64 energies an SM), the rest a warp each where that is less than another wave:
-    // 66 operations a row against 40 with several warps a pipe, so up to about 0.6 of one.  8001 rows: a
-    // wave of pairs 13.0 ms (one thread an energy, all 10000: 34.2 ms; 13.9 with the rest), 5000 energies a
-    // warp each 11.0 ms, 50 energies 1.46 ms (29.0 ms).
     const int sms = pes_sms(), wave = 64 * sms;
     an::PesArgs A{n, dx, dE, Estep, E_start, num_E, 0, 0, V12, rhs0, pes};
     for (int done = 0; done < num_E;) {
         const int left = num_E - done;
-        int np = left * (int64_t)5 > wave * (int64_t)3 && n >= 4 ? (left < wave ? left : wave) : 0;
+        int np = pes_by_pairs(left, n, sms) ? (left < wave ? left : wave) : 0;
+        // a rest for pairs too joins its wave's launch: the SMs that get a second CTA are done no later than
+        // after a second launch (51 rows, 12000 energies: 232 us a call in two launches, 190 in one)
+        if (np == wave && left < 2 * (int64_t)wave && pes_by_pairs(left - wave, n, sms) &&
+            room >= 2 * sizeof(cd) * (size_t)n * left)
+            np = left;
         if (room < 2 * sizeof(cd) * (size_t)n * np) np = 0;
         an::PesPair Q{A, buf, buf + (size_t)n * np, np};
         Q.A.e0 = done;
@@ -442,7 +460,7 @@ extern "C" int mma_tdse_pes(const double* psi, int num_r, double dx, double trg_
         done += np;
         const size_t used = 2 * sizeof(cd) * (size_t)n * np;
         int nw = num_E - done;
-        if (np > 0 && (nw * (int64_t)5 > wave * (int64_t)3 || room < used + 4 * one)) nw = 0;  // the next launch's
+        if (np > 0 && (pes_by_pairs(nw, n, sms) || room < used + 4 * one)) nw = 0;  // the next launch's
         int64_t blocks = (int64_t)((room - used) / (4 * one));
         if (blocks > 4 * sms) blocks = 4 * sms;
         if (blocks > (nw + 3) / 4) blocks = (nw + 3) / 4;
