@@ -13,6 +13,7 @@
 #include "../../include/mma_hankel.h"
 #include "../../include/mma_tdse.h"
 #include "hankel_common.cuh"
+#include "launch.cuh"
 #include "s1tc.cuh"
 #include "tc_sm100.cuh"
 
@@ -975,7 +976,7 @@ int launch_fast(const mma_hankel_problem* p, const mma_hankel_fast_plan_t* plan,
             hi = (float)u;
             lo = (float)(u - (double)hi);
             dim3 g1((unsigned)((p->n_r + kRingR - 1) / kRingR), (unsigned)p->n_omega);
-            cudaFuncSetAttribute(fast_stage1_ring<MM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sr);
+            mma::allow_smem(fast_stage1_ring<MM>);
             fast_stage1_ring<MM><<<g1, kRingR + 32, sr, st>>>(*p, static_cast<const float2*>(src), pre, ptab, ktab,
                                                               rtab, make_float2(hi, lo), Bp, ns, status,
                                                               g_ring_no_issue);
@@ -985,7 +986,7 @@ int launch_fast(const mma_hankel_problem* p, const mma_hankel_fast_plan_t* plan,
         const size_t s1 =
             sizeof(float) * (((size_t)p->n_z * (MM + 4) + 1) / 2 * 2) + sizeof(float2) * (size_t)p->n_z;
         if (s1 > 200 * 1024) return MMA_ERR_TOO_LARGE;
-        cudaFuncSetAttribute(fast_stage1<MM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
+        mma::allow_smem(fast_stage1<MM>);
         dim3 g1((unsigned)((p->n_r + kThreads - 1) / kThreads), (unsigned)p->n_omega);
         fast_stage1<MM><<<g1, kThreads, s1, st>>>(*p, og, rg, src, pre, ptab, Bp);
     }
@@ -1015,11 +1016,11 @@ int launch_fast(const mma_hankel_problem* p, const mma_hankel_fast_plan_t* plan,
         T.c[m] = make_float4(c1, c1, c2, c2);
     }
     if (ser) {
-        cudaFuncSetAttribute(fast_stage2<MM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
+        mma::allow_smem(fast_stage2<MM, true>);
         fast_stage2<MM, true><<<g2, kS2Threads, s2, st>>>(*p, *plan, og, rg, rho, Bp, ff, rtile, asel, vsel, n_sel,
                                                          planes, cut8, cut4, T);
     } else {
-        cudaFuncSetAttribute(fast_stage2<MM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
+        mma::allow_smem(fast_stage2<MM, false>);
         fast_stage2<MM, false><<<g2, kS2Threads, s2, st>>>(*p, *plan, og, rg, rho, Bp, ff, rtile, nullptr, nullptr, 0,
                                                           nullptr, cut8, cut4, T);
     }

@@ -29,6 +29,7 @@
 #include "../../include/mma_hankel.h"
 #include "../../include/mma_tdse.h"
 #include "hankel_common.cuh"
+#include "launch.cuh"
 
 namespace mma {
 namespace hk {
@@ -571,7 +572,7 @@ extern "C" int mma_hankel_plain_ws(const mma_hankel_problem* p, const double* og
     // the nodes of arguments up to about 320 beside A, else what fits
     size_t smem = a_bytes + sizeof(double) * 1300 * kRow;
     if (smem > 220 * 1024) smem = 220 * 1024;
-    if (cudaFuncSetAttribute(direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (mma::allow_smem(direct_kernel) != cudaSuccess)
         return MMA_ERR_CUDA;
     direct_kernel<<<(unsigned)(p->n_omega * jt), kT, smem, st>>>(*p, plan, ogrid, rgrid, zgrid, rho, source, pre2, tab, jt,
                                                                  (int64_t)((smem - a_bytes) / sizeof(double)), ff2, slot,

@@ -24,6 +24,7 @@
 #include "../../include/mma_hankel.h"
 #include "../../include/mma_tdse.h"
 #include "hankel_common.cuh"
+#include "launch.cuh"
 #include "s1tc.cuh"
 #include "tc_sm100.cuh"
 
@@ -374,7 +375,7 @@ int mma::s1tc::stage1_tc_launch(const mma_hankel_problem& P, const void* src, co
     const size_t smem = 1024 + (size_t)kNSrc * kSrcStage + (size_t)kNA * kAStage + (size_t)nkb * 2 * kCTile +
                         (size_t)P.n_z * 16 + 16 * 8;
     if (smem > 227 * 1024) return 0;
-    if (cudaFuncSetAttribute(stage1_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (mma::allow_smem(stage1_tc_kernel) != cudaSuccess)
         return MMA_ERR_CUDA;
     if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return MMA_ERR_CUDA;
     dim3 grid((unsigned)((P.n_r + kRows - 1) / kRows), (unsigned)P.n_omega);

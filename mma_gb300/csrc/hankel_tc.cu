@@ -34,6 +34,7 @@
 #include "../../include/mma_hankel.h"
 #include "../../include/mma_tdse.h"
 #include "hankel_common.cuh"
+#include "launch.cuh"
 #include "tc_sm100.cuh"
 
 namespace mma {
@@ -1048,7 +1049,7 @@ extern "C" int mma_hankel_planes_tc_prepare(const mma_hankel_problem* p, const m
     const int ns = prep_ring_stages(p, source, L);
     if (ns > 0) {
         const size_t sr = prep_ring_smem(L, ns);
-        if (cudaFuncSetAttribute(prep_b_ring, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sr) != cudaSuccess)
+        if (mma::allow_smem(prep_b_ring) != cudaSuccess)
             return MMA_ERR_CUDA;
         prep_b_ring<<<(unsigned)p->n_omega, PREP_THREADS, sr, st>>>(
             *p, make_float2(uh, ul), ogrid, rgrid, reinterpret_cast<const float4*>(sc + L.off_dinv),
@@ -1058,8 +1059,7 @@ extern "C" int mma_hankel_planes_tc_prepare(const mma_hankel_problem* p, const m
         return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
     }
     const size_t sp = sizeof(float2) * (size_t)L.zpad;
-    if (sp > 48 * 1024 &&
-        cudaFuncSetAttribute(prep_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp) != cudaSuccess)
+    if (sp > 48 * 1024 && mma::allow_smem(prep_b) != cudaSuccess)
         return MMA_ERR_CUDA;
     prep_b<<<(unsigned)p->n_omega, PREP_THREADS, sp, st>>>(
         *p, make_float2(uh, ul), ogrid, rgrid, reinterpret_cast<const float4*>(sc + L.off_dinv), source,

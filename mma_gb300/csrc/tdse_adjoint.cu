@@ -18,6 +18,7 @@
 
 #include "../../include/mma_tdse.h"
 #include "common.cuh"
+#include "launch.cuh"
 #include "tdse_cluster.cuh"
 #include "tdse_solver.cuh"
 #include "tdse_step.cuh"
@@ -580,7 +581,7 @@ bool choose_adj_cluster(int max_m, int K, int n_inst, int sms, size_t scratch_by
         if ((size_t)run > scratch_bytes / hist) run = (int)(scratch_bytes / hist);
         if (run > n_inst) run = n_inst;
         if (run < 1 || adj_cluster_us(m, n_inst, run, nc, sms) >= best) continue;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        if (allow_smem(kern) != cudaSuccess ||
             cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
             return false;
         cudaLaunchAttribute at{};
@@ -655,13 +656,13 @@ extern "C" int mma_tdse_adjoint(const mma_tdse_instance* insts, int n_inst, cons
     if (!limited && choose_adj_cluster(max_m, max_ckpt_every, n_inst, sms, bufs->scratch_bytes, &ac)) {
         adj::ClusterArgs Q{A, ac.m, (int64_t)ac.nc * clk::kT * ac.m};
         auto kern = adj::adjoint_cluster_kernel;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ac.smem) != cudaSuccess)
+        if (allow_smem(kern) != cudaSuccess)
             return MMA_ERR_CUDA;
         cudaLaunchAttribute at{};
         cudaLaunchConfig_t cfg = adj_config(ac.nc, ac.clusters, ac.smem, st, &at);
         return cudaLaunchKernelEx(&cfg, kern, Q) == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
     }
-    cudaFuncSetAttribute(adj::adjoint_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(adj::adjoint_fp64_kernel);
     adj::adjoint_fp64_kernel<<<grid_ctas, kThreads, smem, st>>>(A);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }

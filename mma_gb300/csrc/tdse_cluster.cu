@@ -25,6 +25,7 @@
 // (NC = 16), 601 sites 24.3 -> 6.7 us (FP64, NC = 8), 24 float-float instances 35.3 -> 8.8 us.
 #include <cuda_runtime.h>
 
+#include "launch.cuh"
 #include "tdse_cluster.cuh"
 #include "tdse_host.cuh"
 
@@ -369,7 +370,7 @@ template <class N>
 int launch(const clk::Args& A, int nc, int clusters, size_t smem, cudaStream_t st)
 {
     auto k = clk::propagate_cluster_kernel<N>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (allow_smem(k) != cudaSuccess ||
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         return MMA_ERR_CUDA;
     cudaLaunchConfig_t cfg{};
@@ -390,7 +391,7 @@ template <class N>
 int active_clusters(int nc, size_t smem)
 {
     auto k = clk::propagate_cluster_kernel<N>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (allow_smem(k) != cudaSuccess ||
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return 0;

@@ -40,6 +40,7 @@
 #include "../../include/mma_tdse.h"
 #include "common.cuh"
 #include "df64.cuh"
+#include "launch.cuh"
 #include "tdse_step.cuh"
 
 namespace mma {
@@ -472,19 +473,17 @@ extern "C" int mma_tdse_build_df_tables(const mma_tdse_grid* grids_dev, const mm
 
 // CTAs of the float-float form resident at once (two per SM), and the scratch they need:
 // per CTA the sweep buffer and psi, 16 bytes per site each.
-static bool df64_smem_attr(size_t smem)
+static bool df64_smem_attr()
 {
-    return cudaFuncSetAttribute(dfk::propagate_df64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem) == cudaSuccess &&
-           cudaFuncSetAttribute(dfk::propagate_df64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem) == cudaSuccess;
+    return allow_smem(dfk::propagate_df64_kernel<true>) == cudaSuccess &&
+           allow_smem(dfk::propagate_df64_kernel<false>) == cudaSuccess;
 }
 
 extern "C" int mma_tdse_df64_default_ctas()
 {
     int dev = 0, sms = 0, per_sm = 0;
     const size_t smem = dfk::smem_bytes(1);  // up to some thousand sites per thread take no more
-    if (cudaGetDevice(&dev) != cudaSuccess || !df64_smem_attr(smem)) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || !df64_smem_attr()) return 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dfk::propagate_df64_kernel<true>, kThreads, smem);
     return sms * (per_sm > 0 ? per_sm : 1);
@@ -504,7 +503,7 @@ extern "C" int mma_tdse_propagate_df64_impl(const mma_tdse_instance* insts, int 
     dfk::Args A{insts, n_inst, grids, bufs->fields, bufs->outputs, bufs->psi_final, bufs->snapshots, bufs->counter,
                 reinterpret_cast<float4*>(bufs->scratch), (int64_t)max_m * kThreads};
     const size_t smem = dfk::smem_bytes(max_m);
-    if (!df64_smem_attr(smem)) return MMA_ERR_CUDA;
+    if (!df64_smem_attr()) return MMA_ERR_CUDA;
     auto kern = max_m <= dfk::kFlat ? dfk::propagate_df64_kernel<true> : dfk::propagate_df64_kernel<false>;
     kern<<<grid_ctas, kThreads, smem, st>>>(A);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;

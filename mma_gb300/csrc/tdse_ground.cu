@@ -15,6 +15,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include "launch.cuh"
 #include "tdse_host.cuh"
 #include "tdse_solver.cuh"
 #include "tdse_step.cuh"
@@ -252,7 +253,7 @@ bool ground_state_cluster(const mma_tdse_grid* grids_dev, int n_grids, int64_t m
     const size_t smem = sizeof(double) * kVectors * (size_t)m * kT;
     if (smem > (n_grids * kNC > sms ? 110 : 220) * (size_t)1024) return false;
     auto kern = ground_state_cluster_kernel;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
+    if (allow_smem(kern) != cudaSuccess) return false;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(n_grids * kNC));
     cfg.blockDim = dim3(kT * kSub);

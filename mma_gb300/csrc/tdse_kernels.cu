@@ -18,6 +18,7 @@
 
 #include "../../include/mma_tdse.h"
 #include "common.cuh"
+#include "launch.cuh"
 #include "tdse_host.cuh"
 #include "tdse_solver.cuh"
 #include "tdse_step.cuh"
@@ -655,7 +656,7 @@ extern "C" int mma_tdse_default_ctas(int max_m, int precision)
     int per_sm = 1;
     if (psi_fits_smem(max_m)) {
         size_t smem = (size_t)max_m * kThreads * 16;
-        cudaFuncSetAttribute(propagate_fp64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(propagate_fp64_kernel<true>);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, propagate_fp64_kernel<true>, kThreads, smem);
     } else {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, propagate_fp64_kernel<false>, kThreads, 0);
@@ -713,7 +714,7 @@ extern "C" int mma_tdse_propagate_ex(const mma_tdse_instance* insts, int n_inst,
                (double*)bufs->scratch, (int64_t)max_m * kThreads};
     if (psi_fits_smem(max_m)) {
         size_t smem = (size_t)max_m * kThreads * 16;
-        cudaFuncSetAttribute(propagate_fp64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(propagate_fp64_kernel<true>);
         propagate_fp64_kernel<true><<<grid_ctas, kThreads, smem, st>>>(A);
     } else {
         propagate_fp64_kernel<false><<<grid_ctas, kThreads, 0, st>>>(A);
@@ -791,7 +792,7 @@ extern "C" int mma_tdse_propagate_noalloc(const mma_tdse_instance* insts, int n_
                reinterpret_cast<double*>(static_cast<unsigned char*>(base) + kNoAllocHeader),
                (int64_t)max_m * kThreads};
     const size_t smem = per_cta;
-    cudaFuncSetAttribute(propagate_fp64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(propagate_fp64_kernel<true>);
     propagate_fp64_kernel<true><<<ctas, kThreads, smem, st>>>(A);
     return cudaGetLastError() == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
 }
