@@ -27,6 +27,7 @@
 
 #include "../../include/mma_tdse.h"
 #include "dft.cuh"
+#include "launch.cuh"
 
 namespace mma {
 namespace dft {
@@ -757,8 +758,8 @@ int r2c(const Plan* p, const double* x, int64_t xs, double2* X, int64_t Xs, int 
     if (P.threads) return launch_r2c_smem(P, P.threads, x, xs, X, Xs, n_batch, st);
     double2 *a = nullptr, *b = nullptr;
     const size_t bytes = sizeof(double2) * (size_t)P.M * n_batch;
-    if (cudaMallocAsync((void**)&a, bytes, st) != cudaSuccess) return MMA_ERR_CUDA;
-    if (cudaMallocAsync((void**)&b, bytes, st) != cudaSuccess) {
+    if (!succeeded(cudaMallocAsync((void**)&a, bytes, st))) return MMA_ERR_CUDA;
+    if (!succeeded(cudaMallocAsync((void**)&b, bytes, st))) {
         cudaFreeAsync(a, st);
         return MMA_ERR_CUDA;
     }
@@ -803,8 +804,8 @@ int c2r(const Plan* p, const double2* X, int64_t Xs, int n_bins, double* x, int6
     }
     double2 *a = nullptr, *b = nullptr;
     const size_t bytes = sizeof(double2) * (size_t)P.M * n_batch;
-    if (cudaMallocAsync((void**)&a, bytes, st) != cudaSuccess) return MMA_ERR_CUDA;
-    if (cudaMallocAsync((void**)&b, bytes, st) != cudaSuccess) {
+    if (!succeeded(cudaMallocAsync((void**)&a, bytes, st))) return MMA_ERR_CUDA;
+    if (!succeeded(cudaMallocAsync((void**)&b, bytes, st))) {
         cudaFreeAsync(a, st);
         return MMA_ERR_CUDA;
     }

@@ -587,9 +587,8 @@ extern "C" int mma_hankel_plain(const mma_hankel_problem* p, const double* ogrid
     if (!valid(p)) return MMA_ERR_ARG;
     const size_t bytes = mma_hankel_plain_scratch_bytes(p);
     void* ws = nullptr;
-    if (cudaMallocAsync(&ws, bytes, (cudaStream_t)stream) != cudaSuccess) return MMA_ERR_CUDA;
+    if (!mma::succeeded(cudaMallocAsync(&ws, bytes, (cudaStream_t)stream))) return MMA_ERR_CUDA;
     const int rc = mma_hankel_plain_ws(p, ogrid, rgrid, zgrid, rho, source, pre, ff, plane_slot, n_planes, planes, ws,
                                        bytes, stream);
-    if (cudaFreeAsync(ws, (cudaStream_t)stream) != cudaSuccess && rc == MMA_OK) return MMA_ERR_CUDA;
-    return rc;
+    return mma::succeeded(cudaFreeAsync(ws, (cudaStream_t)stream)) ? rc : MMA_ERR_CUDA;
 }

@@ -19,7 +19,16 @@ inline cudaError_t allow_smem(K* kern)
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kern);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+    if (e != cudaSuccess) cudaGetLastError();
     return e;
+}
+
+// False, with the runtime's record of the error cleared, for a call that failed.  The runtime keeps a failure
+// until it is asked for: left there, the next launch's check takes it for its own.
+inline bool succeeded(cudaError_t e)
+{
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
 }
 
 }  // namespace mma

@@ -582,15 +582,12 @@ bool choose_adj_cluster(int max_m, int K, int n_inst, int sms, size_t scratch_by
         if (run > n_inst) run = n_inst;
         if (run < 1 || adj_cluster_us(m, n_inst, run, nc, sms) >= best) continue;
         if (allow_smem(kern) != cudaSuccess ||
-            cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            !succeeded(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)))
             return false;
         cudaLaunchAttribute at{};
         cudaLaunchConfig_t cfg = adj_config(nc, 1, smem, nullptr, &at);
         int active = 0;
-        if (cudaOccupancyMaxActiveClusters(&active, kern, &cfg) != cudaSuccess || active < 1) {
-            cudaGetLastError();
-            continue;
-        }
+        if (!succeeded(cudaOccupancyMaxActiveClusters(&active, kern, &cfg)) || active < 1) continue;
         if (run > active) run = active;
         const double us = adj_cluster_us(m, n_inst, run, nc, sms);
         if (us < best) {
@@ -660,7 +657,7 @@ extern "C" int mma_tdse_adjoint(const mma_tdse_instance* insts, int n_inst, cons
             return MMA_ERR_CUDA;
         cudaLaunchAttribute at{};
         cudaLaunchConfig_t cfg = adj_config(ac.nc, ac.clusters, ac.smem, st, &at);
-        return cudaLaunchKernelEx(&cfg, kern, Q) == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+        return succeeded(cudaLaunchKernelEx(&cfg, kern, Q)) ? MMA_OK : MMA_ERR_CUDA;
     }
     allow_smem(adj::adjoint_fp64_kernel);
     adj::adjoint_fp64_kernel<<<grid_ctas, kThreads, smem, st>>>(A);

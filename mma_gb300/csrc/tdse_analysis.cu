@@ -19,6 +19,7 @@
 #include "../../include/mma_tdse.h"
 #include "common.cuh"
 #include "dft.cuh"
+#include "launch.cuh"
 
 namespace mma {
 namespace an {
@@ -435,7 +436,7 @@ extern "C" int mma_tdse_pes(const double* psi, int num_r, double dx, double trg_
     void* own = nullptr;
     if (room < tabs + 4 * one) {  // a workspace of the least size the call takes: a few warps' worth of its own
         room = tabs + 16 * one;
-        if (cudaMallocAsync(&own, room, st) != cudaSuccess) return MMA_ERR_CUDA;
+        if (!succeeded(cudaMallocAsync(&own, room, st))) return MMA_ERR_CUDA;
         rest = static_cast<char*>(own);
     }
     cd* rhs0t = reinterpret_cast<cd*>(rest);
@@ -474,7 +475,7 @@ extern "C" int mma_tdse_pes(const double* psi, int num_r, double dx, double trg_
         an::pes_kernel<<<(unsigned)(pairs + blocks), 128, 0, st>>>(Q, pairs, W);
     }
     const bool ok = cudaGetLastError() == cudaSuccess;
-    if (own && cudaFreeAsync(own, st) != cudaSuccess) return MMA_ERR_CUDA;
+    if (own && !succeeded(cudaFreeAsync(own, st))) return MMA_ERR_CUDA;
     return ok ? MMA_OK : MMA_ERR_CUDA;
 }
 

@@ -371,7 +371,7 @@ int launch(const clk::Args& A, int nc, int clusters, size_t smem, cudaStream_t s
 {
     auto k = clk::propagate_cluster_kernel<N>;
     if (allow_smem(k) != cudaSuccess ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        !succeeded(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)))
         return MMA_ERR_CUDA;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(clusters * nc));
@@ -384,7 +384,7 @@ int launch(const clk::Args& A, int nc, int clusters, size_t smem, cudaStream_t s
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, A) == cudaSuccess ? MMA_OK : MMA_ERR_CUDA;
+    return succeeded(cudaLaunchKernelEx(&cfg, k, A)) ? MMA_OK : MMA_ERR_CUDA;
 }
 
 template <class N>
@@ -392,10 +392,8 @@ int active_clusters(int nc, size_t smem)
 {
     auto k = clk::propagate_cluster_kernel<N>;
     if (allow_smem(k) != cudaSuccess ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-        cudaGetLastError();
+        !succeeded(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)))
         return 0;
-    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)nc);
     cfg.blockDim = dim3(clk::kT);
@@ -407,11 +405,7 @@ int active_clusters(int nc, size_t smem)
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int c = 0;
-    if (cudaOccupancyMaxActiveClusters(&c, k, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return c;
+    return succeeded(cudaOccupancyMaxActiveClusters(&c, k, &cfg)) ? c : 0;
 }
 
 }  // namespace

@@ -11,6 +11,7 @@
 
 #include "../../include/mma_tdse.h"
 #include "dft.cuh"
+#include "launch.cuh"
 
 namespace {
 
@@ -50,7 +51,7 @@ extern "C" int mma_tdse_prepare_fields(const double* raw, int n_batch, int n_raw
     if (rc == MMA_OK) rc = mma::dft::get_plan(n2, st, &pb);
     if (rc != MMA_OK) return rc;
     double2* spec = nullptr;
-    if (cudaMallocAsync((void**)&spec, sizeof(double2) * (size_t)nc * n_batch, st) != cudaSuccess) return MMA_ERR_CUDA;
+    if (!mma::succeeded(cudaMallocAsync((void**)&spec, sizeof(double2) * (size_t)nc * n_batch, st))) return MMA_ERR_CUDA;
     rc = mma::dft::r2c(pf, raw, n_raw, spec, nc, n_batch, st);
     // the spectrum zero-padded to k1 N / 2 + 1 bins and scaled by 1/N, then the inverse transform
     if (rc == MMA_OK) rc = mma::dft::c2r(pb, spec, nc, nc, interp, n2, n_batch, 1.0 / n_raw, st);
@@ -70,7 +71,7 @@ extern "C" int mma_tdse_spectra(const double* series, int64_t series_stride, int
     int rc = mma::dft::get_plan(n_out, st, &pf);
     if (rc != MMA_OK) return rc;
     double2* spec = nullptr;
-    if (cudaMallocAsync((void**)&spec, sizeof(double2) * (size_t)nc * n_batch, st) != cudaSuccess) return MMA_ERR_CUDA;
+    if (!mma::succeeded(cudaMallocAsync((void**)&spec, sizeof(double2) * (size_t)nc * n_batch, st))) return MMA_ERR_CUDA;
     rc = mma::dft::r2c(pf, series, series_stride, spec, nc, n_batch, st);
     if (rc == MMA_OK) {
         const double two_pi = 6.283185307179586476925286766559;

@@ -247,25 +247,40 @@ __global__ void __launch_bounds__(kT* kSub) ground_state_cluster_kernel(const mm
 
 }  // namespace
 
-bool ground_state_cluster(const mma_tdse_grid* grids_dev, int n_grids, int64_t m, int sms, cudaStream_t st)
+namespace {
+cudaLaunchConfig_t config(int n_grids, int64_t m, cudaStream_t st, cudaLaunchAttribute* at)
 {
-    // all clusters resident at once, for n_grids up to a quarter of the SMs (the caller's rule)
-    const size_t smem = sizeof(double) * kVectors * (size_t)m * kT;
-    if (smem > (n_grids * kNC > sms ? 110 : 220) * (size_t)1024) return false;
-    auto kern = ground_state_cluster_kernel;
-    if (allow_smem(kern) != cudaSuccess) return false;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(n_grids * kNC));
     cfg.blockDim = dim3(kT * kSub);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = sizeof(double) * kVectors * (size_t)m * kT;
     cfg.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kNC;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = kNC;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, grids_dev, (int)m) == cudaSuccess;
+    return cfg;
+}
+}  // namespace
+
+bool ground_state_fits(int n_grids, int64_t m, int sms)
+{
+    if (n_grids * 4 > sms) return false;
+    // all clusters resident at once, two CTAs an SM where they are more than the SMs
+    if (sizeof(double) * kVectors * (size_t)m * kT > (n_grids * kNC > sms ? 110 : 220) * (size_t)1024) return false;
+    cudaLaunchAttribute at{};
+    const cudaLaunchConfig_t cfg = config(n_grids, m, nullptr, &at);
+    int active = 0;
+    return allow_smem(ground_state_cluster_kernel) == cudaSuccess &&
+           succeeded(cudaOccupancyMaxActiveClusters(&active, ground_state_cluster_kernel, &cfg)) && active > 0;
+}
+
+bool ground_state_cluster(const mma_tdse_grid* grids_dev, int n_grids, int64_t m, cudaStream_t st)
+{
+    cudaLaunchAttribute at{};
+    const cudaLaunchConfig_t cfg = config(n_grids, m, st, &at);
+    return succeeded(cudaLaunchKernelEx(&cfg, ground_state_cluster_kernel, grids_dev, (int)m));
 }
 
 }  // namespace mma

@@ -22,9 +22,11 @@ bool choose_cluster(int max_m, int precision, int n_inst, int sms, ClusterPlan* 
 int launch_cluster(const ClusterPlan& p, const mma_tdse_instance* insts, int n_inst, const mma_tdse_grid* grids,
                    const mma_tdse_buffers* bufs, int max_m, int precision, void* stream);
 
-// The ground states of a few grids by a cluster each, from the tables and V that build_grids_kernel mode 3
-// left; false (and nothing launched) where a CTA per grid serves better (tdse_ground.cu).
-bool ground_state_cluster(const mma_tdse_grid* grids_dev, int n_grids, int64_t max_m, int sms, cudaStream_t st);
+// The ground states of a few grids by a cluster each (tdse_ground.cu).  Whether a cluster serves these grids
+// (else a CTA each does), and the launch, from the tables and V that build_grids_kernel mode 3 left: false,
+// and nothing launched, where it fails.
+bool ground_state_fits(int n_grids, int64_t max_m, int sms);
+bool ground_state_cluster(const mma_tdse_grid* grids_dev, int n_grids, int64_t max_m, cudaStream_t st);
 // x and the ground state of one grid, without its Crank-Nicolson tables (tdse_kernels.cu)
 int ground_state_only(const mma_tdse_grid* grid_dev, int64_t m, cudaStream_t st);
 

@@ -602,10 +602,9 @@ static int sm_count()
 // x and the ground states of grids with their tables: by a cluster per grid where they are few
 static bool few_ground_states(const mma_tdse_grid* grids_dev, int n_grids, int64_t max_m, cudaStream_t st)
 {
-    const int sms = sm_count();
-    if (n_grids * 4 > sms) return false;
+    if (!ground_state_fits(n_grids, max_m, sm_count())) return false;
     build_grids_kernel<<<n_grids, kThreads, 0, st>>>(grids_dev, 3);
-    return ground_state_cluster(grids_dev, n_grids, max_m, sms, st);
+    return ground_state_cluster(grids_dev, n_grids, max_m, st);
 }
 
 int mma::ground_state_only(const mma_tdse_grid* grid_dev, int64_t m, cudaStream_t st)
