@@ -121,6 +121,11 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_fp64_kernel(Args P)
         const double* ai = P.a + P.a_off[inst];
         double* gi = P.grad + P.grad_off[inst];
         const double dt = G.dt, dx = G.dx;
+        if (L > P.max_L || K > P.max_K) {  // wider than the launch was sized for: a NaN gradient
+            for (int64_t e = t; e < S; e += kThreads) gi[e] = __longlong_as_double(0x7ff8000000000000LL);
+            __syncthreads();
+            continue;
+        }
         if (t == 0) s_gate = gate_index(f, I.n_field, S, I.gate_floor);
         for (int64_t i = 0; i < m; i++) lam[i * kThreads + t] = cd{0.0, 0.0};  // lambda_S = 0
         __syncthreads();

@@ -190,6 +190,13 @@ __global__ void __launch_bounds__(kThreads, 2) propagate_df64_kernel(Args P)
         double *o_t = out, *o_e = out + (S + 1), *o_src = out + 2 * (S + 1), *o_ptot = out + 3 * (S + 1),
                *o_pint = out + 4 * (S + 1), *o_x = out + 5 * (S + 1);
         const double dt = G.dt, dx = G.dx;
+        if (L > P.max_L) {
+            // a grid wider than the launch was sized for would overrun this CTA's buffers and the factors in
+            // shared memory: NaN outputs, as in the FP64 kernel
+            for (int64_t e = t; e < 6 * (S + 1); e += kThreads) out[e] = __longlong_as_double(0x7ff8000000000000LL);
+            __syncthreads();
+            continue;
+        }
         if (t == 0) {
             s_gate = gate_index(f, I.n_field, S, I.gate_floor);
             const int64_t num_r = n - 1;  // PopInt window (tools_algorithmic.c:19-43)
