@@ -137,7 +137,9 @@ __global__ void __launch_bounds__(kT) plan_kernel(mma_hankel_problem P, const do
         const double x = 0.5 * sg * km * rm * hm / d_ref;
         const double M = terms_for(x);
         const double two = 80.0 * P.n_z + 2.0 * M * P.n_z + (30.0 + 6.0 * M) * P.n_rho, one = 17.0 * (double)P.n_z * P.n_rho;
-        out->series = n_planes <= kSel && bad == 0.0 && x <= kCut[kTerms] && want < (double)kNodes && two < one;
+        // distances whose squares leave the range of doubles (infinity too) have no reference distance
+        const bool range = dn < 1e150 && dx < 1e150;
+        out->series = n_planes <= kSel && bad == 0.0 && range && x <= kCut[kTerms] && want < (double)kNodes && two < one;
     }
 }
 
