@@ -363,10 +363,13 @@ __global__ void __launch_bounds__(T) r2c_smem(Plan P, const double* __restrict__
 // Windowed magnitudes g[row][k] = norm |r2c(win[row % n_win] * sig[row / n_win])_k|, k < nf: the window on
 // the way in, the magnitude on the way out, and only the bins asked for formed in the last pass and the
 // unpacking (the Gabor transform asks for a sixth of them).  Bound by the FP64 pipe: 4410 samples, 352
-// bins, 51200 rows: 15.2 ms as r2c with 1.0 ms of passes around it, 12.3 ms here.
-constexpr int kWinT = 384;  // 95 registers a thread leave one CTA of 512 an SM: 13.3 ms against 12.3
+// bins, 51200 rows: 15.2 ms as r2c with 1.0 ms of passes around it, 12.2 ms here.  T: rows of up to 1024
+// values take 256 threads, longer ones 384 (64 samples, 6400 rows: 107 us with 256 threads, 152 with 384, 283
+// with 512; 4410 samples, 352 bins, 51200 rows: 12.27, 12.20 and 13.25 ms, 10 rows 53, 50 and 50 us).
+constexpr int kShortRow = 1024;
 
-__global__ void __launch_bounds__(kWinT) windowed_smem(Plan P, const double* __restrict__ sig, int64_t stride,
+template <int T>
+__global__ void __launch_bounds__(T) windowed_smem(Plan P, const double* __restrict__ sig, int64_t stride,
                                                    const double* __restrict__ win, int n_win, int nf, double norm,
                                                    double* __restrict__ g, int64_t n_batch)
 {
@@ -375,7 +378,7 @@ __global__ void __launch_bounds__(kWinT) windowed_smem(Plan P, const double* __r
     const int t = threadIdx.x;
     for (int64_t row = blockIdx.x; row < n_batch; row += gridDim.x) {
         const double *xr = sig + row / n_win * stride, *wr = win + row % n_win * P.n;
-        for (int j = t; j < P.M; j += kWinT) {
+        for (int j = t; j < P.M; j += T) {
             double2 z = make_double2(0.0, 0.0);
             if (j < P.L) {
                 if (P.n % 2 == 0) z = make_double2(wr[2 * j] * xr[2 * j], wr[2 * j + 1] * xr[2 * j + 1]);
@@ -388,14 +391,14 @@ __global__ void __launch_bounds__(kWinT) windowed_smem(Plan P, const double* __r
         double2* Z;
         if (P.bluestein) {
             Z = fft_smem(b0, b1, P);
-            for (int j = t; j < P.M; j += kWinT) Z[j] = conjg(cmul(Z[j], __ldg(P.bker + j)));
+            for (int j = t; j < P.M; j += T) Z[j] = conjg(cmul(Z[j], __ldg(P.bker + j)));
             __syncthreads();
             Z = fft_smem_part(Z, Z == b0 ? b1 : b0, P, nf);
         } else {
             Z = fft_smem_part(b0, b1, P, nf);
         }
         auto at = [&](int k) { return P.bluestein ? cmul(conjg(Z[k]), __ldg(P.chirp + k)) : Z[k]; };
-        for (int k = t; k < nf; k += kWinT) {
+        for (int k = t; k < nf; k += T) {
             double2 v = at(k == P.L ? 0 : k);
             if (P.n % 2 == 0) v = r2c_out(P, v, conjg(at(k == 0 ? 0 : P.L - k)), k);
             g[row * nf + k] = norm * sqrt(v.x * v.x + v.y * v.y);
@@ -603,7 +606,8 @@ int set_smem_attrs()
         cudaFuncSetAttribute(c2r_smem<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
         cudaFuncSetAttribute(r2c_smem<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
         cudaFuncSetAttribute(c2r_smem<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
-        cudaFuncSetAttribute(windowed_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+        cudaFuncSetAttribute(windowed_smem<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(windowed_smem<384>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
         return MMA_ERR_CUDA;
     if (dev >= 0 && dev < 64) done[dev] = 1;
     return MMA_OK;
@@ -781,10 +785,20 @@ bool windowed(const Plan* p, const double* sig, int64_t stride, int n_sig, const
 {
     const Plan& P = *p;
     if (!P.threads) return false;
+    // Long rows of an even length with most of their bins wanted: unpacking the bins and their square roots serve
+    // better as passes of their own, over all SMs.  us here / in passes for half, three quarters and all of the
+    // bins: 4410 samples, 10 rows 62, 66, 72 / 64, 64, 64, 6400 rows 1971, 2183, 2380 / 2189, 2259, 2330; 3528
+    // samples, 6400 rows 1541, 1711, 1858 / 1570, 1626, 1681; 7000 samples 3135, 3453, 3799 / 3418, 3527, 3639.
+    // So from half of them on for fewer rows than two waves of CTAs, else from three quarters on.  An odd
+    // length has no unpacking (2205: 1740 / 1783 for all), and rows of up to kShortRow values gain here with
+    // every bin (1764 samples, 800 rows: 142 / 159).
     const int64_t n = (int64_t)n_sig * n_win;
+    if (P.M > kShortRow && P.n % 2 == 0 && 4 * (int64_t)nf > (n <= 304 ? 2 : 3) * (int64_t)(P.n / 2 + 1)) return false;
     const int b = (int)(n < (1 << 20) ? n : (1 << 20));
     const size_t smem = 2 * (size_t)P.M * sizeof(double2);
-    windowed_smem<<<b, kWinT, smem, st>>>(P, sig, stride, win, n_win, nf, norm, g, n);
+    const int threads = P.M <= kShortRow ? 256 : 384;
+    auto k = threads == 256 ? windowed_smem<256> : windowed_smem<384>;
+    k<<<b, threads, smem, st>>>(P, sig, stride, win, n_win, nf, norm, g, n);
     return true;
 }
 

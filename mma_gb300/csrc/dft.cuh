@@ -30,7 +30,8 @@ int r2c(const Plan* p, const double* x, int64_t x_stride, double2* X, int64_t X_
         cudaStream_t st);
 
 // norm |r2c(win_w sig_s)_k| for k < nf into g[s n_win + w][nf] (signals at sig + s stride, windows [n_win][n],
-// nf <= n/2 + 1) where rows fit in shared memory; false, and nothing launched, where they do not.
+// nf <= n/2 + 1) where rows fit in shared memory; false, and nothing launched, where they do not or where
+// passes of their own are faster.
 bool windowed(const Plan* p, const double* sig, int64_t stride, int n_sig, const double* win, int n_win, int nf,
               double norm, double* g, cudaStream_t st);
 
