@@ -49,7 +49,6 @@ __constant__ double kCut[kTerms + 1] = {
 struct Plan {
     double d_ref, sigma, k_max, r_max, rho_max, d_min, u_max;
     double selw[kSel][kTerms];     // (1 - lambda^2)^m / m! of the selected planes
-    int sel_kz[kSel];
     int nodes, series;
 };
 
@@ -112,7 +111,6 @@ __global__ void __launch_bounds__(kT) plan_kernel(mma_hankel_problem P, const do
         }
         if (slot && slot[i] >= 0 && slot[i] < kSel) {
             c = 1.0;
-            out->sel_kz[slot[i]] = (int)i;
 #pragma unroll
             for (int m = 0; m < kTerms; m++) {
                 out->selw[slot[i]][m] = c;
