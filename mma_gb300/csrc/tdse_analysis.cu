@@ -385,7 +385,7 @@ int pes_sms()
 {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 1;
+    return sms > 0 ? sms : 152;  // sizes can be asked for without a device
 }
 
 // Whether pairs serve `left` energies (or the first wave of them, 64 energies an SM) of n rows sooner than a
@@ -411,11 +411,12 @@ extern "C" size_t mma_tdse_pes_scratch_bytes(int num_r, int chunk)
     const size_t n = (size_t)num_r + 1, m = (n + 31) / 32;
     // the pairs' two arrays of `chunk` energies, then gamma, y and f of the energies that a warp each
     // takes: those beyond full waves of pairs, as many as run at once (16 warps an SM)
-    const size_t wave = 64 * 152, left = (size_t)chunk % wave;
-    const size_t rest = left > 0 && !pes_by_pairs((int64_t)left, (int64_t)n, 152) ? left : 0;
+    const int sms = pes_sms();
+    const size_t wave = 64 * (size_t)sms, left = (size_t)chunk % wave;
+    const size_t rest = left > 0 && !pes_by_pairs((int64_t)left, (int64_t)n, sms) ? left : 0;
     const size_t warps = ((size_t)chunk < wave ? (size_t)chunk : rest) + 3;
     return pes_fixed(n) + 32 * m * 24 + 512 + 2 * sizeof(cd) * n * ((size_t)chunk - rest) +
-           48 * 32 * m * ((warps < 16 * 152 ? warps : 16 * 152) / 4 * 4);
+           48 * 32 * m * ((warps < 16 * (size_t)sms ? warps : 16 * (size_t)sms) / 4 * 4);
 }
 
 extern "C" int mma_tdse_pes(const double* psi, int num_r, double dx, double trg_a, int num_E, double dE, double Estep,
