@@ -176,7 +176,6 @@ __global__ void __launch_bounds__(kT* kSub) ground_state_cluster_kernel(const mm
         send_edges();
         cluster.sync();
         // ---- energy quotient (tridiag.c:172-238): the terms by all warps, each chunk's sum by its own
-#pragma unroll 1  // unrolled, the compiled loop of an earlier form summed two of three sites at m = 3
         for (int i = sub; i < m; i += kSub) {
             const int q = i * kT + lane;
             const double pm = i > 0 ? psi[q - kT] : lane == 0 ? S.left : psi[(m - 1) * kT + lane - 1];
