@@ -23,8 +23,11 @@ __device__ __forceinline__ double minus_grad_v(double x, double a)
 
 // (K psi) and (M2 psi) at site i of a thread's m in the energy quotient (tridiag.c:172-238).  The inverse
 // iteration stops on this quotient's rounding, so its last bit decides how often it runs and with that
-// psi0's twelfth digit: every fused operation is spelled out.  Which of the neighbours' two products is
-// fused alternates by pairs of sites, as it always has.
+// psi0's twelfth digit.  Every fused operation is therefore spelled out, for the one-CTA and the cluster
+// kernel alike.  Which of the neighbours' two products is fused has no meaning in the mathematics: any fixed
+// choice is as good.  The alternation by pairs of sites keeps the bits that grids have had since the
+// quotient was a loop unrolled by four, and with them the results that depend on psi0's last bit: complex64
+// propagation carries one changed bit of psi0 into 2e-5 of its outputs (its own rounding), FP64 into 1e-11.
 __device__ __forceinline__ void quotient_terms(double inv_dx2, double pm, double pc, double pn, double vm, double vc,
                                                double vn, int i, int m, double& kpsi, double& mpsi)
 {
