@@ -189,8 +189,8 @@ def run_config0(args, device):
            "legacy_fp64": {"seconds_per_call": float(np.median(secs)), "calls": len(secs),
                            "site_steps_per_s": site_steps / float(np.median(secs)),
                            "rel_l2_vs_reference": errs(r),
-                           "note": "wall clock of the PythonCTDSE-surface call: ground state, one CTA "
-                                   "propagating, spectra, host copies"}}
+                           "note": "wall clock of the PythonCTDSE-surface call: ground state, propagation "
+                                   "over a cluster of CTAs, spectra, host copies"}}
     dtf = float(t[1] - t[0])
     grids = TDSEGrids([dict(num_r=num_r, dx=dx, trg_a=a)], dt=dtf, df64=True)
     Ed = torch.tensor(E[None, :], device=device)

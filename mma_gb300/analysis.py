@@ -1,7 +1,7 @@
 """Batched TDSE analysis on the GPU: photoelectron spectra and Gabor transforms.
 
-``pes`` computes window_analysis (1DTDSE/sources/tools.c:206-316) for many energies at once, one
-GPU thread per energy; ``gabor`` computes GaborTransform (1DTDSE/sources/tools_fftw3.c:158-213)
+``pes`` computes window_analysis (1DTDSE/sources/tools.c:206-316) for many energies at once, by a pair
+of GPU threads or a warp per energy; ``gabor`` computes GaborTransform (1DTDSE/sources/tools_fftw3.c:158-213)
 for a batch of signals (for example every instance's dipole acceleration of a TDSE batch).
 Inputs and outputs are torch tensors on the GPU; the kernels are in csrc/tdse_analysis.cu.
 The reference's single-call host forms are ``TDSE_DLL.compute_PES`` / ``gabor_transform``.

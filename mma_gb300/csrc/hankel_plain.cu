@@ -10,8 +10,10 @@
 //   * J0 (and J1) come from Taylor sums of 12 terms about nodes 1/4 apart (|d| <= 1/8, truncation
 //     (1/8)^11/11! = 3e-18 in J1), whose coefficients follow from J0 and J1 at the node by Bessel's
 //     equation x y'' + y' + x y = 0.  The table (112 bytes a node) is made once per call.  11 FMAs
-//     a J0 against about 147 FP64 operations a term with CUDA's j0 (measured), at the same accuracy:
-//     both are within 1e-16 rms of J0 on [0, 330].  Arguments beyond the table's nodes take j0.
+//     a J0 against about 147 FP64 operations a term with CUDA's j0 (measured).  The far field is within
+//     1.3e-16 of its largest value of extended-precision sums (64 planes x 512 r, arguments up to 330), where
+//     sums with CUDA's j0, itself up to 1.1e-13 off there, were within 1.1e-15.  Arguments beyond the
+//     table's nodes take j0.
 //   * Where at most two planes are wanted for themselves, FF contracts z first through the
 //     multiplication theorem J0(lambda y) = sum_m (1 - lambda^2)^m / m! G_m(y), G_m = (y/2)^m J_m(y),
 //     lambda = d_ref/D_k: B_m[w, r] = sum_k tau_k (1 - lambda_k^2)^m / m! A_k, then
@@ -141,8 +143,8 @@ __global__ void __launch_bounds__(kT) plan_kernel(mma_hankel_problem P, const do
     }
 }
 
-// J0 and J1 at a node to rounding (CUDA's j1 is 1e-12 off beyond x = 8, which a Taylor sum would carry
-// into every value about the node): below 25 Miller's backward recurrence normalised by
+// J0 and J1 at a node to rounding (CUDA's j1 is up to 4.4e-13 off on [25, 330], which a Taylor sum would
+// carry into every value about the node): below 25 Miller's backward recurrence normalised by
 // J0 + 2 (J2 + J4 + ...) = 1 (Abramowitz & Stegun 9.12), above it Hankel's asymptotic series
 // (9.2.5-9.2.10), whose smallest term there is e^{-2x} = 2e-22.
 __device__ void bessel01(double x, double& J0, double& J1)

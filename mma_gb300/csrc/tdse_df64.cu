@@ -30,8 +30,8 @@
 // threads for some twenty steps at a time, and the observables' warp sums stay double-word until lanes
 // of warp 0 convert them.
 //
-// Bound by the double-word chains' latency and the CTA barriers between the passes (FMA pipe 49% busy,
-// issue 46%, a quarter of the warps' time at barriers).  Per step of 304 instances of 8001 sites (two CTAs
+// Bound by the double-word chains' latency and the CTA barriers between the passes (304 instances, 884 steps:
+// FMA pipe 60% busy, issue 54%, an eighth of the warps' time at barriers).  Per step of 304 instances of 8001 sites (two CTAs
 // an SM): 58.9 us before the operand ring was aligned, the chunks kept their own frames (below), the
 // correction and the backward sweep became one sum and a real psi0 took half a projection; 54.0 us now
 // with 11% fewer instructions.  The whole benchmark map, 4 cycles: 667 -> 609 ms.
