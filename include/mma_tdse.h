@@ -239,7 +239,8 @@ typedef struct mma_tdse_buffers {
 } mma_tdse_buffers;
 
 /* Build x, -V', ground state and the solve tables of n_grids grids (device array
- * `grids_dev`, host copy `grids_host` for validation).  One CTA per grid.
+ * `grids_dev`, host copy `grids_host` for validation).  One CTA per grid; the ground states
+ * of few grids by a cluster of CTAs each, with the same bits.
  * mode 0: everything; mode 1: CN tables only, from the x and psi0 already in the
  * grid's buffers (a caller-supplied ground state). */
 int mma_tdse_build_grids(const mma_tdse_grid *grids_dev, const mma_tdse_grid *grids_host, int n_grids, int mode,
@@ -252,10 +253,12 @@ int mma_tdse_build_grids(const mma_tdse_grid *grids_dev, const mma_tdse_grid *gr
 int mma_tdse_build_c64_tables(const mma_tdse_grid *grids_dev, const mma_tdse_grid *grids_host, int n_grids,
                               void *stream);
 
-/* Propagate n_inst instances in one persistent launch (one CTA per instance at a
- * time, instances pulled from a device work queue).
+/* Propagate n_inst instances in one persistent launch (instances pulled from a device work
+ * queue, each by one CTA or, in FP64 and float-float where that finishes the batch sooner, by
+ * a cluster of CTAs).  An instance on a grid wider than max_m gets NaN outputs.
  *   max_m      largest grid m in the batch (sizes shared memory and scratch)
- *   grid_ctas  persistent CTAs to launch (0 = as many as are resident at once)
+ *   grid_ctas  persistent CTAs to launch (0 = as many as are resident at once); fewer than
+ *              that and than n_inst keeps one CTA per instance and the limit
  *   precision  0 = FP64, the reference's arithmetic;
  *              1 = complex64 propagation (FP32 wavefunction and sweeps) with the
  *                  factorisation computed in FP64 and the observables summed with
@@ -290,10 +293,11 @@ int mma_tdse_c64_shape_ok(int cta_threads, int m32);
  * m32 <= 16, one otherwise); 0 for a shape without a kernel. */
 int mma_tdse_c64_default_ctas(int m32, int cta_threads);
 
-/* Photoelectron spectra on the GPU (window_analysis's algorithm, device pointers): one thread
- * per energy, two FP64 Numerov-tridiagonal solves each.  psi [2(num_r+1)] interleaved, pes
- * [num_E].  Scratch: the energies run in chunks of as many as the scratch holds;
- * mma_tdse_pes_scratch_bytes(num_r, chunk) is the size for `chunk` energies at a time. */
+/* Photoelectron spectra on the GPU (window_analysis's algorithm, device pointers): two threads
+ * or a warp per energy, two FP64 Numerov-tridiagonal solves each.  psi [2(num_r+1)] interleaved,
+ * pes [num_E].  Scratch: the energies run in chunks of as many as the scratch holds;
+ * mma_tdse_pes_scratch_bytes(num_r, chunk) is the size for `chunk` energies at a time.  A scratch
+ * that holds one energy is enough: the call then takes its own from the stream-ordered allocator. */
 size_t mma_tdse_pes_scratch_bytes(int num_r, int chunk);
 int mma_tdse_pes(const double *psi, int num_r, double dx, double trg_a, int num_E, double dE, double Estep,
                  double E_start, double *pes, void *scratch, size_t scratch_bytes, void *stream);
